@@ -42,6 +42,7 @@
 #include "bulk_copy.cuh"
 #include "gpu_ops.h"
 #include "lina_gpu.h"
+#include "strip_solve.cuh"
 
 namespace {
 
@@ -300,11 +301,22 @@ __global__ void __launch_bounds__(kWinThreads, 1) sptrsv_window_kernel(const Win
             bulk::mbar_drain(bars + (l % S), (unsigned)((l / S) & 1), kWaitNs);
 }
 
+// any NaN becomes the canonical one (tested by its bits: an FP64 comparison would take the slow FP64 pipe).
+// FP64 arithmetic hands on the sign and payload of a NaN operand, so operands free of other NaNs keep the
+// strips' results free of the pending pattern.
+__device__ __forceinline__ float plain_nan(float v) {
+    return (__float_as_uint(v) & 0x7fffffffu) > 0x7f800000u ? __uint_as_float(Word<float>::kNaN) : v;
+}
+__device__ __forceinline__ double plain_nan(double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    return u > 0x7ff0000000000000ull ? __longlong_as_double((long long)Word<double>::kNaN) : v;
+}
+
 // bpos[t] = b[row[t]] (0 on padding positions): the right-hand side in position order
-template <typename TX>
-__global__ void gather_pos_kernel(int n, const int* __restrict__ row, const TX* __restrict__ b, TX* __restrict__ bpos) {
+template <typename TB, typename TX>
+__global__ void gather_pos_kernel(int n, const int* __restrict__ row, const TB* __restrict__ b, TX* __restrict__ bpos) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-        bpos[t] = row[t] >= 0 ? b[row[t]] : TX(0);
+        bpos[t] = row[t] >= 0 ? plain_nan(TX(b[row[t]])) : TX(0);
 }
 
 // x[row[t]] = xpos[t]: the solution from position order (padding positions skipped)
@@ -322,6 +334,27 @@ __global__ void pack_values_kernel(long ne, const int* __restrict__ perm, const 
         const int p = perm[q];  // -1: padding
         w64[q] = p >= 0 ? v64[p] : 0.0;
         w32[q] = p >= 0 ? v32[p] : 0.0f;
+    }
+}
+
+// the strips' packed entries (place in shared memory in bytes, factor value) and positions (row, 1/L_ii or 1)
+__global__ void strip_entries_kernel(long ne, const int* __restrict__ enc, const int* __restrict__ perm,
+                                     const double* __restrict__ v64, const float* __restrict__ v32,
+                                     strip::Entry<double>* __restrict__ e64, strip::Entry<float>* __restrict__ e32) {
+    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < ne; q += (long)gridDim.x * blockDim.x) {
+        const int p = perm[q], at = enc[q];  // p -1: padding
+        e64[q] = strip::Entry<double>{8u * at, 0u, p >= 0 ? plain_nan(v64[p]) : 0.0};
+        e32[q] = strip::Entry<float>{4u * at, p >= 0 ? plain_nan(v32[p]) : 0.0f};
+    }
+}
+
+__global__ void strip_points_kernel(int n, const int* __restrict__ row, const double* __restrict__ d64,
+                                    const float* __restrict__ d32, strip::Point<double>* __restrict__ p64,
+                                    strip::Point<float>* __restrict__ p32) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int i = row[t];
+        p64[t] = strip::Point<double>{i, 0, i >= 0 && d64 ? plain_nan(d64[i]) : 1.0};
+        p32[t] = strip::Point<float>{i, i >= 0 && d32 ? plain_nan(d32[i]) : 1.0f};
     }
 }
 
@@ -549,6 +582,18 @@ struct Factor {
         double *val64 = nullptr, *dinv64 = nullptr;
         float *val32 = nullptr, *dinv32 = nullptr;
     } win;
+    // the solve pipelined over strips (strips = 0: one of the other two)
+    struct Strips {
+        int strips = 0, ring = 0, width = 0, max_width = 0;
+        int npos = 0;
+        long ne = 0;
+        int *first = nullptr, *ext_first = nullptr, *ext = nullptr, *table = nullptr, *row = nullptr;
+        int *enc = nullptr, *perm = nullptr;
+        strip::Entry<double>* entry64 = nullptr;
+        strip::Entry<float>* entry32 = nullptr;
+        strip::Point<double>* point64 = nullptr;
+        strip::Point<float>* point32 = nullptr;
+    } strip;
 };
 
 struct Mem {
@@ -748,6 +793,18 @@ void plan_window(WinPlan& pl, int n, const std::vector<int>& order, const std::v
     if (w.s64) w.smem64 = win_smem<double, double>(ring, max_rows, max_ent, has_dinv, w.s64);
 }
 
+// the position-major work vectors, shared by both factors and both kinds of plan
+bool ensure_positions(lina_gpu_ilu* h, int npos) {
+    if (h->npos >= npos) return true;
+    Mem& m = h->mem;
+    h->bpos64 = m.get<double>(npos);
+    h->xpos64 = m.get<double>(npos);
+    h->bpos32 = m.get<float>(npos);
+    h->xpos32 = m.get<float>(npos);
+    h->npos = npos;
+    return h->bpos64 && h->xpos64 && h->bpos32 && h->xpos32;
+}
+
 // the plan's arrays on the device; a factor without a plan (levels too wide or too large) keeps
 // the row pool
 bool upload_window(lina_gpu_ilu* h, Factor& f, const WinPlan& pl, bool has_dinv) {
@@ -768,14 +825,7 @@ bool upload_window(lina_gpu_ilu* h, Factor& f, const WinPlan& pl, bool has_dinv)
         w.dinv32 = m.get<float>(w.npos);
         ok = ok && w.dinv64 && w.dinv32;
     }
-    if (ok && h->npos < w.npos) {  // position-major work vectors, shared by both factors
-        h->bpos64 = m.get<double>(w.npos);
-        h->xpos64 = m.get<double>(w.npos);
-        h->bpos32 = m.get<float>(w.npos);
-        h->xpos32 = m.get<float>(w.npos);
-        ok = h->bpos64 && h->xpos64 && h->bpos32 && h->xpos32;
-        h->npos = w.npos;
-    }
+    ok = ok && ensure_positions(h, w.npos);
     if (!ok) {
         w = Factor::Win();
         return false;
@@ -783,24 +833,77 @@ bool upload_window(lina_gpu_ilu* h, Factor& f, const WinPlan& pl, bool has_dinv)
     return true;
 }
 
-bool build_window(lina_gpu_ilu* h, Factor& f, int n, const std::vector<int>& order, const std::vector<int>& lev,
-                  const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end,
-                  const int* col, bool has_dinv) {
-    WinPlan pl;
-    plan_window(pl, n, order, lev, lp, beg, end, col, has_dinv);
-    return upload_window(h, f, pl, has_dinv);
+// How a factor is solved: pipelined over strips where its plan exists (strip::make_plan says which
+// matrices suit it), else by one block walking the levels where a level fits its shared memory, else by
+// the row pool.  ILU(0) of the AT2 damage matrix on GB300, one application (two solves):
+//   1025 x 1025 nodes, FP32: one block 2.87 ms, strips 0.52 ms
+//    389 x 389 nodes, FP64: one block 1.20 ms, strips 0.45 ms
+struct SolvePlan {
+    strip::Plan strips;
+    WinPlan window;
+};
+
+void plan_solve(SolvePlan& pl, int n, const std::vector<int>& order, const std::vector<int>& lev,
+                const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end, const int* col,
+                bool has_dinv, bool lower) {
+    if (!strip::make_plan(pl.strips, n, order, lev, (int)lp.size() - 1, beg, end, col, lower))
+        plan_window(pl.window, n, order, lev, lp, beg, end, col, has_dinv);
 }
 
-// the window's packed copies of a factor's values and inverse diagonal (after every factorisation)
-void pack_window(Factor& f, int n) {
+bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl, bool has_dinv) {
+    const strip::Plan& p = pl.strips;
+    if (!p.strips) return upload_window(h, f, pl.window, has_dinv);
+    Factor::Strips& w = f.strip;
+    Mem& m = h->mem;
+    w = Factor::Strips();
+    w.ring = p.ring;
+    w.width = p.width;
+    w.max_width = p.max_width;
+    w.npos = (int)p.positions();
+    w.ne = p.entries();
+    w.first = m.up(p.first);
+    w.ext_first = m.up(p.ext_first);
+    w.ext = m.up(p.ext);
+    w.table = m.up(p.table);
+    w.row = m.up(p.row);
+    w.enc = m.up(p.enc);
+    w.perm = m.up(p.perm);
+    w.entry64 = m.get<strip::Entry<double>>(w.ne);
+    w.entry32 = m.get<strip::Entry<float>>(w.ne);
+    w.point64 = m.get<strip::Point<double>>(w.npos);
+    w.point32 = m.get<strip::Point<float>>(w.npos);
+    bool ok = w.first && w.ext_first && w.ext && w.table && w.row && w.enc && w.perm && w.entry64 &&
+              w.entry32 && w.point64 && w.point32;
+    ok = ok && ensure_positions(h, w.npos);
+    if (ok) w.strips = p.strips;
+    return ok;
+}
+
+bool build_solve(lina_gpu_ilu* h, Factor& f, int n, const std::vector<int>& order, const std::vector<int>& lev,
+                 const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end,
+                 const int* col, bool has_dinv, bool lower) {
+    SolvePlan pl;
+    plan_solve(pl, n, order, lev, lp, beg, end, col, has_dinv, lower);
+    return upload_solve(h, f, pl, has_dinv);
+}
+
+// the solve plan's packed copies of a factor's values and inverse diagonal (after every factorisation)
+void pack_solve(Factor& f, int n) {
+    if (f.strip.strips) {
+        Factor::Strips& w = f.strip;
+        const int ge = (int)std::min<long>(4096, (w.ne + kT - 1) / kT), gp = std::min(4096, (w.npos + kT - 1) / kT);
+        strip_entries_kernel<<<ge, kT, 0, st()>>>(w.ne, w.enc, w.perm, f.val64, f.val32, w.entry64, w.entry32);
+        strip_points_kernel<<<gp, kT, 0, st()>>>(w.npos, w.row, f.dinv64, f.dinv32, w.point64, w.point32);
+        return;
+    }
     Factor::Win& w = f.win;
     if (!w.s32 && !w.s64) return;
     pack_values_kernel<<<std::min<long>(4096, (w.ne + kT - 1) / kT), kT, 0, st()>>>(w.ne, w.vperm, f.val64, f.val32,
                                                                                    w.val64, w.val32);
     if (w.dinv64) {
         const int g = std::min(4096, (w.npos + kT - 1) / kT);
-        gather_pos_kernel<double><<<g, kT, 0, st()>>>(w.npos, w.row, f.dinv64, w.dinv64);
-        gather_pos_kernel<float><<<g, kT, 0, st()>>>(w.npos, w.row, f.dinv32, w.dinv32);
+        gather_pos_kernel<double, double><<<g, kT, 0, st()>>>(w.npos, w.row, f.dinv64, w.dinv64);
+        gather_pos_kernel<float, float><<<g, kT, 0, st()>>>(w.npos, w.row, f.dinv32, w.dinv32);
     }
 }
 
@@ -862,11 +965,11 @@ bool build_factor(lina_gpu_ilu* h, Factor& f, int n, const int* p, const int* c,
     }
     f.beg = dptr;
     f.end = dptr + 1;
-    if (!build_window(h, f, n, order, lev, lp, beg, end, col.data(), !unit)) {
+    if (!build_solve(h, f, n, order, lev, lp, beg, end, col.data(), !unit, lower)) {
         err = "device allocation for the ILU factors failed";
         return false;
     }
-    pack_window(f, n);
+    pack_solve(f, n);
     return true;
 }
 
@@ -890,8 +993,8 @@ int factorise(lina_gpu_ilu* h) {
     diag_inverse_kernel<<<std::min(4096, (n + kT - 1) / kT), kT, 0, st()>>>(n, h->adiag, h->fval, h->L.dinv64,
                                                                              h->L.dinv32);
     cvt_kernel<double, float><<<std::min<long>(4096, (nnz + kT - 1) / kT), kT, 0, st()>>>(nnz, h->fval, h->L.val32);
-    pack_window(h->L, n);
-    pack_window(h->U, n);
+    pack_solve(h->L, n);
+    pack_solve(h->U, n);
     const int e = (cudaGetLastError() == cudaSuccess) ? read_err(h) : -1;
     if (e != 0) {
         lina::dev::set_error(e == 2 ? "ILU: zero pivot (incomplete_LU_factorization fails)"
@@ -922,8 +1025,70 @@ void launch_window(lina_gpu_ilu* h, const Factor& f, const WinArgs<TV, TX>& a, s
         launch_window_t<TV, TX, S, false>(a, smem);
 }
 
+template <typename TX, int EM, bool DINV>
+void launch_strips_t(const strip::Args<TX>& a, int strips, size_t smem) {
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(strip::solve_kernel<TX, EM, DINV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             strip::kSmemMax);
+        attr = true;
+    }
+    strip::solve_kernel<TX, EM, DINV><<<strips, strip::kThreads, smem, st()>>>(a);
+}
+
+template <typename TX, int EM>
+void launch_strips(const strip::Args<TX>& a, int strips, size_t smem, bool dinv) {
+    if (dinv)
+        launch_strips_t<TX, EM, true>(a, strips, smem);
+    else
+        launch_strips_t<TX, EM, false>(a, strips, smem);
+}
+
+// the solve pipelined over strips; the right-hand side may be wider than the solve's type
+template <typename TX, typename TB>
+void solve_strips(lina_gpu_ilu* h, const Factor& f, const TX* dinv, const TB* b, TX* x) {
+    const Factor::Strips& w = f.strip;
+    strip::Args<TX> a;
+    a.ring = w.ring;
+    a.max_width = w.max_width;
+    a.stages = strip::stages_for(w.ring, w.max_width, sizeof(TX));
+    a.first = w.first;
+    a.ext_first = w.ext_first;
+    a.ext = w.ext;
+    a.table = reinterpret_cast<const int4*>(w.table);
+    TX* bpos;
+    if constexpr (sizeof(TX) == 8) {
+        a.entry = w.entry64;
+        a.point = w.point64;
+        bpos = h->bpos64;
+    } else {
+        a.entry = w.entry32;
+        a.point = w.point32;
+        bpos = h->bpos32;
+    }
+    a.b = bpos;
+    a.x = x;
+    a.ticket = h->ticket;
+    a.err = h->err;
+    gather_pos_kernel<TB, TX><<<std::min(4096, (w.npos + kT - 1) / kT), kT, 0, st()>>>(w.npos, w.row, b, bpos);
+    cudaMemsetAsync(x, 0xff, (size_t)h->n * sizeof(TX), st());  // every entry pending
+    cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
+    const size_t smem = strip::smem_bytes(w.ring, w.max_width, sizeof(TX), a.stages);
+    switch (w.width) {
+        case 1: launch_strips<TX, 1>(a, w.strips, smem, dinv != nullptr); break;
+        case 2: launch_strips<TX, 2>(a, w.strips, smem, dinv != nullptr); break;
+        case 3: launch_strips<TX, 3>(a, w.strips, smem, dinv != nullptr); break;
+        case 4: launch_strips<TX, 4>(a, w.strips, smem, dinv != nullptr); break;
+        default: launch_strips<TX, 0>(a, w.strips, smem, dinv != nullptr); break;
+    }
+}
+
 template <typename TV, typename TX>
 void solve(lina_gpu_ilu* h, const Factor& f, const TV* val, const TX* dinv, const TX* b, TX* x) {
+    if (f.strip.strips) {
+        solve_strips<TX, TX>(h, f, dinv, b, x);
+        return;
+    }
     const int n = h->n;
     const Factor::Win& w = f.win;
     const int stages = sizeof(TX) == 8 ? w.s64 : w.s32;
@@ -951,7 +1116,7 @@ void solve(lina_gpu_ilu* h, const Factor& f, const TV* val, const TX* dinv, cons
         a.bpos = bpos;
         a.err = h->err;
         const int g = std::min(4096, (w.npos + kT - 1) / kT);
-        gather_pos_kernel<TX><<<g, kT, 0, st()>>>(w.npos, w.row, b, bpos);
+        gather_pos_kernel<TX, TX><<<g, kT, 0, st()>>>(w.npos, w.row, b, bpos);
         const size_t smem = sizeof(TX) == 8 ? w.smem64 : w.smem32;
         switch (stages) {
             case 6: launch_window<TV, TX, 6>(h, f, a, smem); break;
@@ -1033,16 +1198,16 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
     h->fnnz = nnz;
     std::vector<int> lorder, uorder, llev, ulev, llp, ulp;
     lap("pattern checks and splits");
-    // the level schedules and window plans of L and U are independent: U's on a second thread
-    WinPlan lplan, uplan;
+    // the level schedules and solve plans of L and U are independent: U's on a second thread
+    SolvePlan lplan, uplan;
     std::thread upper([&] {
         h->U.nlev = level_order(n, ubeg, uend, col, false, uorder, &ulev, &ulp);
-        plan_window(uplan, n, uorder, ulev, ulp, ubeg, uend, col, false);
+        plan_solve(uplan, n, uorder, ulev, ulp, ubeg, uend, col, false, false);
     });
     h->L.nlev = level_order(n, lbeg, lend, col, true, lorder, &llev, &llp);
-    plan_window(lplan, n, lorder, llev, llp, lbeg, lend, col, true);
+    plan_solve(lplan, n, lorder, llev, llp, lbeg, lend, col, true, true);
     upper.join();
-    lap("level schedules and window plans");
+    lap("level schedules and solve plans");
     Mem& m = h->mem;
     int *dptr = nullptr, *dcol = nullptr, *ddiag = nullptr;
     double* dval = nullptr;
@@ -1074,7 +1239,7 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
     h->L.col = h->U.col = dcol;
     h->L.val64 = h->U.val64 = h->fval;
     h->U.val32 = h->L.val32;
-    if (!upload_window(h, h->L, lplan, true) || !upload_window(h, h->U, uplan, false)) {
+    if (!upload_solve(h, h->L, lplan, true) || !upload_solve(h, h->U, uplan, false)) {
         lina::dev::set_error("ILU: device allocation failed");
         delete h;
         return LINA_GPU_ECUDA;
@@ -1089,7 +1254,7 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
         delete h;
         return LINA_GPU_ECUDA;
     }
-    lap("window uploads");
+    lap("solve plan uploads");
     const int rc = factorise(h);
     if (rc) {
         delete h;
@@ -1175,8 +1340,12 @@ int lina_gpu_ilu_apply(lina_gpu_ilu* h, int precision, const double* r_dev, doub
     const int n = h->n;
     const int g = (int)std::min<long>(2048, (n + kT - 1) / kT);
     if (precision == LINA_PREC_MIXED) {
-        cvt_kernel<double, float><<<g, kT, 0, st()>>>(n, r_dev, h->r32);
-        solve<float, float>(h, h->L, h->L.val32, h->L.dinv32, h->r32, h->t32);
+        if (h->L.strip.strips) {
+            solve_strips<float, double>(h, h->L, h->L.dinv32, r_dev, h->t32);
+        } else {
+            cvt_kernel<double, float><<<g, kT, 0, st()>>>(n, r_dev, h->r32);
+            solve<float, float>(h, h->L, h->L.val32, h->L.dinv32, h->r32, h->t32);
+        }
         solve<float, float>(h, h->U, h->U.val32, h->U.dinv32, h->t32, h->z32);
         cvt_kernel<float, double><<<g, kT, 0, st()>>>(n, h->z32, z_dev);
     } else {

@@ -1,0 +1,183 @@
+// strip_plan.h - host side of the strip-pipelined triangular solves (strip_solve.cuh): which matrices suit
+// them, and the layout of the strips' steps.
+#pragma once
+
+#include <algorithm>
+#include <cstddef>
+#include <cstdint>
+#include <vector>
+
+namespace strip {
+
+constexpr int kSteps = 8;                  // steps per chunk (one stage of shared memory)
+constexpr int kPos = 32 * kSteps;          // positions per chunk
+constexpr int kHelpers = 2;                // helper warps
+constexpr int kThreads = 32 * (2 + kHelpers);
+constexpr int kRingMin = 16, kRingMax = 64;  // steps a strip keeps in shared memory: more than a chunk
+constexpr int kSlots = 512;                // hand-over slots: the fetched entries of two chunks fit
+constexpr int kMaxStrips = 148;            // one block per SM, a few left free
+constexpr int kRowsPerStrip = 30;          // rows of the widest level per strip: a step holds 32
+constexpr int kMaxEntries = 16;            // entries of a row (stage size)
+constexpr int kSmemMax = 200 * 1024;
+constexpr int kLag = 25;                   // steps an exchange between strips takes (about 2 us)
+
+// The plan of one factor: positions are chunk * 256 + step * 32 + lane.
+struct Plan {
+    int strips = 0;      // 0: the matrix does not suit the strips
+    int chunks = 0;
+    int ring = 0;        // steps kept (a power of two)
+    int width = 0;       // entries per row of every chunk where that is at most 4, else 0 (table)
+    int max_width = 0;
+    std::vector<int> first;            // first chunk of each strip (strips + 1)
+    std::vector<int> ext_first;        // first fetched entry of each strip (strips + 1)
+    std::vector<int> ext;              // row of each fetched entry
+    std::vector<int> table;            // per chunk: offset of its entries, entries per row, end of its fetched entries, 0
+    std::vector<int> row;              // row of each position, -1 none
+    std::vector<int> enc, perm;        // per entry: the place of its operand in shared memory; its value's index
+    long entries() const { return (long)enc.size(); }
+    size_t positions() const { return (size_t)chunks * kPos; }
+};
+
+// Rows listed level by level (order, with lev[i] the level of row i, nlev levels), row i's entries
+// [beg_i, end_i) of col.  lower: a row needs smaller indices.  Returns false (no plan) where
+//  - the widest level has more than 4,440 rows: the levels are wide enough for the other solves;
+//  - a row has more than 16 entries (stages of shared memory);
+//  - more than 8 entries per step come from other strips, which the helper warps could not fetch in
+//    the time of a step (64 lanes, an L2 round trip each);
+//  - a chunk has more than 256 fetched entries (it and the next one share the slots);
+//  - the pipeline, followed step by step, takes more than 4 steps per level: a step is about 0.05 us in
+//    FP32 and 0.15 us in FP64, a level of the one-block solve 0.3 us and more.
+inline bool make_plan(Plan& P, int n, const std::vector<int>& order, const std::vector<int>& lev, int nlev,
+                      const std::vector<int>& beg, const std::vector<int>& end, const int* col, bool lower) {
+    P = Plan();
+    if (n <= 0 || nlev <= 0) return false;
+    std::vector<int> width(nlev, 0);
+    int maxw = 0, maxe = 1;
+    for (int i = 0; i < n; i++) {
+        maxw = std::max(maxw, ++width[lev[i]]);
+        maxe = std::max(maxe, end[i] - beg[i]);
+    }
+    if (maxw > kMaxStrips * kRowsPerStrip || maxe > kMaxEntries) return false;
+    const int K = std::max(1, std::min(n, (maxw + kRowsPerStrip - 1) / kRowsPerStrip));
+    auto strip_of = [&](int i) { return (int)((long)(lower ? i : n - 1 - i) * K / n); };
+    // rows by strip, then level
+    std::vector<int> start(K + 1, 0), rows(n), stepof(n);
+    for (int i = 0; i < n; i++) start[strip_of(i) + 1]++;
+    for (int s = 0; s < K; s++) start[s + 1] += start[s];
+    {
+        std::vector<int> at(start.begin(), start.end() - 1);
+        for (int t = 0; t < n; t++) rows[at[strip_of(order[t])]++] = order[t];
+    }
+    // steps: up to 32 rows of one level; stepof = step within the strip * 32 + lane
+    std::vector<int> nsteps(K, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int s = 0; s < K; s++) {
+        int step = -1, lane = 32, level = -1;
+        for (int t = start[s]; t < start[s + 1]; t++) {
+            const int i = rows[t];
+            if (lane == 32 || lev[i] != level) {
+                step++;
+                lane = 0;
+                level = lev[i];
+            }
+            stepof[i] = step * 32 + lane++;
+        }
+        nsteps[s] = step + 1;
+    }
+    // how far back a strip's rows reach within it
+    int look = 1;
+#pragma omp parallel for schedule(static) reduction(max : look)
+    for (int i = 0; i < n; i++)
+        for (int p = beg[i]; p < end[i]; p++)
+            if (strip_of(col[p]) == strip_of(i)) look = std::max(look, stepof[i] / 32 - stepof[col[p]] / 32);
+    P.ring = kRingMin;
+    while (P.ring < look + 1 && P.ring < kRingMax) P.ring *= 2;
+    const int ring = P.ring;
+    auto fetched = [&](int i, int j) {
+        return strip_of(i) != strip_of(j) || stepof[i] / 32 - stepof[j] / 32 >= ring;
+    };
+    P.first.assign(K + 1, 0);
+    for (int s = 0; s < K; s++) P.first[s + 1] = P.first[s] + (nsteps[s] + kSteps - 1) / kSteps;
+    P.chunks = P.first[K];
+    P.max_width = maxe;
+    P.width = maxe <= 4 ? maxe : 0;
+    // entries per row of every chunk
+    P.table.assign(4 * (size_t)P.chunks, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int s = 0; s < K; s++)
+        for (int t = start[s]; t < start[s + 1]; t++) {
+            int& w = P.table[4 * (size_t)(P.first[s] + stepof[rows[t]] / kPos) + 1];
+            w = P.width ? P.width : std::max(w, end[rows[t]] - beg[rows[t]]);
+        }
+    long total = 0, steps = 0;
+    for (int c = 0; c < P.chunks; c++) {
+        P.table[4 * (size_t)c] = (int)total;
+        total += (long)P.table[4 * (size_t)c + 1] * kPos;
+        if (total > INT32_MAX / 2) return false;
+    }
+    for (int s = 0; s < K; s++) steps += nsteps[s];
+    if (P.positions() > (size_t)INT32_MAX / 2) return false;
+    const int empty = ring * 32 + kSlots;  // a word that holds zero, for padding
+    P.row.assign(P.positions(), -1);
+    P.enc.assign(total, empty);
+    P.perm.assign(total, -1);
+    std::vector<std::vector<int>> ext(K), ext_step(K);
+#pragma omp parallel for schedule(dynamic, 1)
+    for (int s = 0; s < K; s++) {
+        int t = start[s];
+        std::vector<int>& x = ext[s];
+        for (int step = 0; step < nsteps[s]; step++) {
+            int t1 = t;
+            while (t1 < start[s + 1] && stepof[rows[t1]] / 32 == step) t1++;
+            const int c = P.first[s] + step / kSteps;
+            const size_t at = (size_t)P.table[4 * (size_t)c] + 32 * (size_t)(step % kSteps);
+            for (int u = t; u < t1; u++) P.row[(size_t)c * kPos + 32 * (size_t)(step % kSteps) + (u - t)] = rows[u];
+            for (int k = 0; k < P.table[4 * (size_t)c + 1]; k++)  // fetched entries are numbered entry by entry
+                for (int u = t; u < t1; u++) {
+                    const int i = rows[u], p = beg[i] + k;
+                    if (p >= end[i]) continue;
+                    const size_t q = at + (size_t)k * kPos + (u - t);
+                    P.perm[q] = p;
+                    if (fetched(i, col[p])) {
+                        P.enc[q] = ring * 32 + (int)(x.size() % kSlots);
+                        x.push_back(col[p]);
+                        ext_step[s].push_back(step);
+                    } else {
+                        P.enc[q] = (stepof[col[p]] / 32 % ring) * 32 + stepof[col[p]] % 32;
+                    }
+                }
+            t = t1;
+            P.table[4 * (size_t)c + 2] = (int)x.size();
+        }
+    }
+    for (int s = 0; s < K; s++)
+        for (int c = P.first[s]; c < P.first[s + 1]; c++)
+            if (P.table[4 * (size_t)c + 2] - (c == P.first[s] ? 0 : P.table[4 * (size_t)c - 2]) > kSlots / 2) return false;
+    P.ext_first.assign(K + 1, 0);
+    for (int s = 0; s < K; s++) P.ext_first[s + 1] = P.ext_first[s] + (int)ext[s].size();
+    P.ext.resize(P.ext_first[K]);
+    for (int s = 0; s < K; s++) std::copy(ext[s].begin(), ext[s].end(), P.ext.begin() + P.ext_first[s]);
+    if ((long)P.ext.size() > 8 * steps) return false;
+    // the pipeline in units of a step: a step starts when the one before it and its chunk's fetched entries are
+    // there
+    std::vector<std::vector<long>> done(K);
+    long last = 0;
+    for (int s = 0; s < K; s++) {
+        done[s].assign(nsteps[s], 0);
+        size_t e = 0;
+        long now = 0;
+        for (int step = 0; step < nsteps[s]; step++) {
+            for (; e < ext[s].size() && ext_step[s][e] / kSteps == step / kSteps; e++) {
+                const int j = ext[s][e];
+                now = std::max(now, done[strip_of(j)][stepof[j] / 32] + kLag);
+            }
+            done[s][step] = ++now;
+        }
+        last = std::max(last, now);
+    }
+    if (last > 4L * nlev + 4L * kLag) return false;
+    P.strips = K;
+    return true;
+}
+
+}  // namespace strip
