@@ -42,7 +42,7 @@
 #include "bulk_copy.cuh"
 #include "gpu_ops.h"
 #include "lina_gpu.h"
-#include "strip_solve.cuh"
+#include "strip_factor.cuh"
 
 namespace {
 
@@ -683,6 +683,14 @@ struct lina_gpu_ilu {
     int *aptr = nullptr, *acol = nullptr, *adiag = nullptr;  // A's pattern (device factorisation)
     double* aval = nullptr;                                  // A's values
     long fnnz = 0;
+    // the factorisation pipelined over strips (width 0: the row pool)
+    struct StripFactor {
+        int width = 0, ring = 0, strips = 0, npos = 0;
+        unsigned used = 0;
+        int *ext_first = nullptr, *ext = nullptr, *ext_end = nullptr, *rec = nullptr;
+        short* place = nullptr;
+        double* a = nullptr;
+    } sf;
 };
 
 namespace {
@@ -981,6 +989,52 @@ int read_err(lina_gpu_ilu* h) {
     return e;
 }
 
+// A's values of every position's row, laid out as strip::factor_kernel reads them (padding: 0, on the diagonal 1)
+template <int W>
+__global__ void strip_rows_kernel(int npos, const int2* __restrict__ rec, const double* __restrict__ val,
+                                  double* __restrict__ a) {
+    constexpr int NE = 2 * W + 1;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npos; t += gridDim.x * blockDim.x) {
+        const int2 r = rec[t];
+        const int nlow = r.y & 0xff, nup = r.y >> 8;
+        double* out = a + (size_t)(t / strip::kPos) * strip::kPos * NE + t % strip::kPos;
+#pragma unroll
+        for (int e = 0; e < NE; e++) {
+            const int k = e - (W - nlow);  // the row's k-th entry
+            double v = e == W ? 1.0 : 0.0;
+            if (r.x >= 0 && k >= 0 && k <= nlow + nup) v = plain_nan(val[r.x + k]);
+            out[(size_t)e * strip::kPos] = v;
+        }
+    }
+}
+
+template <int W>
+void launch_strip_factor(lina_gpu_ilu* h) {
+    const lina_gpu_ilu::StripFactor& w = h->sf;
+    strip::FactorArgs a;
+    a.ring = w.ring;
+    a.stages = strip::factor_stages(W, w.ring);
+    a.used = w.used;
+    a.first = h->L.strip.first;
+    a.ext_first = w.ext_first;
+    a.ext = w.ext;
+    a.ext_end = w.ext_end;
+    a.rec = reinterpret_cast<const int2*>(w.rec);
+    a.place = w.place;
+    a.a = w.a;
+    a.f = h->fval;
+    a.ticket = h->ticket;
+    a.err = h->err;
+    static bool attr = false;
+    if (!attr) {
+        cudaFuncSetAttribute(strip::factor_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, strip::kSmemMax);
+        attr = true;
+    }
+    strip_rows_kernel<W><<<std::min(4096, (w.npos + kT - 1) / kT), kT, 0, st()>>>(w.npos, a.rec, h->aval, w.a);
+    cudaMemsetAsync(h->fval, 0xff, (size_t)h->fnnz * sizeof(double), st());  // every entry pending
+    strip::factor_kernel<W><<<w.strips, strip::factor_threads(W), strip::factor_smem(W, w.ring, a.stages), st()>>>(a);
+}
+
 // ILU(0) of the handle's A (pattern and values on the device) into fval, the inverse diagonal and
 // the FP32 copy of the factors; each factorisation is a new pass of the row flags
 int factorise(lina_gpu_ilu* h) {
@@ -988,8 +1042,15 @@ int factorise(lina_gpu_ilu* h) {
     const long nnz = h->fnnz;
     h->epoch++;
     cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
-    ilu0_kernel<<<pool_blocks(n), kPool, 0, st()>>>(n, h->L.order, h->aptr, h->acol, h->aval, h->adiag, h->U.beg,
-                                                    h->fval, h->flag, h->epoch, h->ticket, h->err);
+    switch (h->sf.width) {
+        case 1: launch_strip_factor<1>(h); break;
+        case 2: launch_strip_factor<2>(h); break;
+        case 3: launch_strip_factor<3>(h); break;
+        case 4: launch_strip_factor<4>(h); break;
+        default:
+            ilu0_kernel<<<pool_blocks(n), kPool, 0, st()>>>(n, h->L.order, h->aptr, h->acol, h->aval, h->adiag, h->U.beg,
+                                                            h->fval, h->flag, h->epoch, h->ticket, h->err);
+    }
     diag_inverse_kernel<<<std::min(4096, (n + kT - 1) / kT), kT, 0, st()>>>(n, h->adiag, h->fval, h->L.dinv64,
                                                                              h->L.dinv32);
     cvt_kernel<double, float><<<std::min<long>(4096, (nnz + kT - 1) / kT), kT, 0, st()>>>(nnz, h->fval, h->L.val32);
@@ -1206,6 +1267,8 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
     });
     h->L.nlev = level_order(n, lbeg, lend, col, true, lorder, &llev, &llp);
     plan_solve(lplan, n, lorder, llev, llp, lbeg, lend, col, true, true);
+    strip::FactorPlan fplan;
+    strip::make_factor_plan(fplan, lplan.strips, n, rowptr, col, diag);
     upper.join();
     lap("level schedules and solve plans");
     Mem& m = h->mem;
@@ -1243,6 +1306,25 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
         lina::dev::set_error("ILU: device allocation failed");
         delete h;
         return LINA_GPU_ECUDA;
+    }
+    if (fplan.width) {
+        lina_gpu_ilu::StripFactor& w = h->sf;
+        w.width = fplan.width;
+        w.used = fplan.used;
+        w.ring = lplan.strips.ring;
+        w.strips = lplan.strips.strips;
+        w.npos = (int)lplan.strips.positions();
+        w.ext_first = m.up(fplan.ext_first);
+        w.ext = m.up(fplan.ext);
+        w.ext_end = m.up(fplan.ext_end);
+        w.rec = m.up(fplan.rec);
+        w.place = m.up(fplan.place);
+        w.a = m.get<double>((size_t)w.npos * (2 * w.width + 1));
+        if (!w.ext_first || !w.ext || !w.ext_end || !w.rec || !w.place || !w.a) {
+            lina::dev::set_error("ILU: device allocation failed");
+            delete h;
+            return LINA_GPU_ECUDA;
+        }
     }
     h->flag = m.get<int>(n);
     h->aptr = dptr;

@@ -7,6 +7,12 @@
 #include <cstdint>
 #include <vector>
 
+#ifdef __CUDACC__
+#define STRIP_HD __host__ __device__
+#else
+#define STRIP_HD
+#endif
+
 namespace strip {
 
 constexpr int kSteps = 8;                  // steps per chunk (one stage of shared memory)
@@ -177,6 +183,127 @@ inline bool make_plan(Plan& P, int n, const std::vector<int>& order, const std::
     }
     if (last > 4L * nlev + 4L * kLag) return false;
     P.strips = K;
+    return true;
+}
+
+// ---------------------------------------------------------------- the ILU(0) factorisation on the strips
+// A row of the factorisation needs the upper entries U_kj of the rows k its lower entries name: the
+// dependencies of the lower solve, so its steps are walked.  A row's entries are held as W lower ones (as
+// many padding ones first as it has fewer), the diagonal and W upper ones; a "pair" is a product
+// L_ik U_kj of a lower entry k (slot q) in the sum of a later entry j (a lower slot > q, the diagonal, an
+// upper slot).  The pairs are numbered by entry, then by q, the order in which the sums take them.
+constexpr int kFactorWidth = 4;
+STRIP_HD constexpr int pairs_of(int W) { return W * (W - 1) / 2 + W + W * W; }
+STRIP_HD constexpr int pair_index(int W, int entry, int q) {  // entry: lower slot, W the diagonal, W + 1 + t an upper slot
+    return entry < W ? entry * (entry - 1) / 2 + q : W * (W - 1) / 2 + (entry - W) * W + q;
+}
+
+// Quotients a / d of one row share the reciprocal of d.  Markstein's method ("Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990): with r = 1 / d rounded to nearest, a q within a few ulps of
+// a / d is corrected by its exact remainder, q + (a - d q) r; the second correction rounds as the quotient
+// does.  Only for exponents within +-400 of 0 (or a = 0, where a r has the right sign), so that no remainder
+// loses bits; exponents are looked at as integers.
+STRIP_HD inline bool mid_range(unsigned high_word) {
+    const unsigned e = (high_word >> 20) & 0x7ffu;
+    return e >= 1023u - 400u && e <= 1023u + 400u;
+}
+
+struct FactorPlan {
+    int width = 0;                // 0: none
+    unsigned used = 0;            // pairs that some row has
+    std::vector<int> rec;         // per position: first entry of the row in CSR, lower entries | upper entries << 8
+    std::vector<short> place;     // per chunk and pair: where U_kj is in shared memory, -1 none
+    std::vector<int> ext_first, ext;  // fetched entries: the CSR entry of U_kj
+    std::vector<int> ext_end;     // per chunk: end of its fetched entries within its strip's
+};
+
+// On the lower factor's plan.  False where a row has more than four entries on either side of the diagonal or
+// none on it, or where the fetched entries of a chunk exceed the slots.
+inline bool make_factor_plan(FactorPlan& F, const Plan& P, int n, const int* ptr, const int* col,
+                             const std::vector<int>& diag) {
+    F = FactorPlan();
+    if (!P.strips || !P.width) return false;
+    int W = 1, bad = 0;
+#pragma omp parallel for schedule(static) reduction(max : W) reduction(| : bad)
+    for (int i = 0; i < n; i++) {
+        if (diag[i] < 0) bad = 1;
+        W = std::max(W, std::max(diag[i] - ptr[i], ptr[i + 1] - 1 - diag[i]));
+    }
+    if (bad || W > kFactorWidth) return false;
+    const int NP = pairs_of(W), rw = P.ring * 32;
+    std::vector<int> pos(n);  // chunk * 256 + step * 32 + lane
+#pragma omp parallel for schedule(static)
+    for (size_t t = 0; t < P.positions(); t++)
+        if (P.row[t] >= 0) pos[P.row[t]] = (int)t;
+    F.rec.assign(2 * P.positions(), 0);
+    for (size_t t = 0; t < P.positions(); t++)
+        if (P.row[t] < 0) F.rec[2 * t] = -1;
+    F.place.assign(P.positions() * NP, -1);
+    F.ext_end.assign(P.chunks, 0);
+    F.ext_first.assign(P.strips + 1, 0);
+    std::vector<std::vector<int>> ext(P.strips);
+    unsigned used = 0;
+#pragma omp parallel for schedule(dynamic, 1) reduction(| : used, bad)
+    for (int s = 0; s < P.strips; s++) {
+        std::vector<int>& x = ext[s];
+        const int lo = P.first[s] * kPos, hi = P.first[s + 1] * kPos;
+        for (int c = P.first[s]; c < P.first[s + 1]; c++) {
+            const size_t before = x.size();
+            for (int st = 0; st < kSteps; st++) {
+                int src[pairs_of(kFactorWidth)][32];  // per pair and lane: the CSR entry of U_kj
+                for (int k = 0; k < NP; k++)
+                    for (int l = 0; l < 32; l++) src[k][l] = -1;
+                const size_t p0 = (size_t)c * kPos + 32 * (size_t)st;
+                for (int l = 0; l < 32; l++) {
+                    const int i = P.row[p0 + l];
+                    if (i < 0) continue;
+                    const int r0 = ptr[i], d = diag[i], r1 = ptr[i + 1], nlow = d - r0;
+                    F.rec[2 * (p0 + l)] = r0;
+                    F.rec[2 * (p0 + l) + 1] = nlow | (r1 - 1 - d) << 8;
+                    for (int a = r0; a < d; a++) {
+                        const int k = col[a], q = W - nlow + (a - r0);
+                        int e = a + 1;
+                        for (int u = diag[k] + 1; u < ptr[k + 1]; u++) {
+                            while (e < r1 && col[e] < col[u]) e++;
+                            if (e == r1) break;
+                            if (col[e] != col[u]) continue;
+                            const int entry = e < d ? W - nlow + (e - r0) : W + (e - d);
+                            src[pair_index(W, entry, q)][l] = u;
+                        }
+                    }
+                }
+                for (int k = 0; k < NP; k++)
+                    for (int l = 0; l < 32; l++) {
+                        const int u = src[k][l];
+                        if (u < 0) continue;
+                        used |= 1u << k;
+                        // the row that u belongs to is the lower entry's column
+                        int r = 0;
+                        {
+                            const int i = P.row[p0 + l], d = diag[i];
+                            for (int a = ptr[i]; a < d; a++)
+                                if (u > diag[col[a]] && u < ptr[col[a] + 1]) r = col[a];
+                        }
+                        const size_t at = (size_t)c * kPos * NP + (size_t)k * kPos + 32 * (size_t)st + l;
+                        const int back = (int)((p0 - lo) / 32) - (pos[r] - lo) / 32;
+                        if (pos[r] >= lo && pos[r] < hi && back < P.ring) {
+                            F.place[at] = (short)((u - diag[r] - 1) * rw + (pos[r] - lo) % rw);
+                        } else {
+                            F.place[at] = (short)(W * rw + (int)(x.size() % kSlots));
+                            x.push_back(u);
+                        }
+                    }
+            }
+            if (x.size() - before > kSlots / 2) bad = 1;
+            F.ext_end[c] = (int)x.size();
+        }
+    }
+    if (bad || W * rw + kSlots > 32767) return false;
+    for (int s = 0; s < P.strips; s++) F.ext_first[s + 1] = F.ext_first[s] + (int)ext[s].size();
+    F.ext.resize(F.ext_first[P.strips]);
+    for (int s = 0; s < P.strips; s++) std::copy(ext[s].begin(), ext[s].end(), F.ext.begin() + F.ext_first[s]);
+    F.used = used;
+    F.width = W;
     return true;
 }
 

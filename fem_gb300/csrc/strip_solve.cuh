@@ -164,55 +164,64 @@ __device__ __forceinline__ bool keep_waiting(long& polls, unsigned long long& t0
 // the helper warps: fetched entry e of the strip goes to slot e mod kSlots once its row is solved and the
 // slot is empty.  One loop for all lanes, each at an entry of its own: a lane that waits holds up no other.
 template <typename TX>
-__device__ void fetch_entries(const Args<TX>& a, int strip, int lane, unsigned char* slots) {
+__device__ void fetch_entries(const TX* x, const int* __restrict__ ext, int e0, int e1, int lane, unsigned char* slots,
+                              int* err) {
     using B = Bits<TX>;
     using U = typename B::U;
-    const int e1 = __ldg(a.ext_first + strip + 1), e0 = __ldg(a.ext_first + strip);
     int e = e0 + lane;
-    int src = e < e1 ? __ldg(a.ext + e) : 0;
-    int nsrc = e + 32 * kHelpers < e1 ? __ldg(a.ext + e + 32 * kHelpers) : 0;
+    int src = e < e1 ? __ldg(ext + e) : 0;
+    int nsrc = e + 32 * kHelpers < e1 ? __ldg(ext + e + 32 * kHelpers) : 0;
     U u = B::kPending;
     long polls = 0;
     unsigned long long t0 = 0;
     while (e < e1) {
         unsigned char* slot = slots + (e - e0) % kSlots * (int)sizeof(TX);
-        if (u == B::kPending) u = B::poll(a.x + src);
+        if (u == B::kPending) u = B::poll(x + src);
         if (u != B::kPending && get<TX>(slot) == B::kPending) {
             put<TX>(slot, u);
             u = B::kPending;
             e += 32 * kHelpers;
             src = nsrc;
-            nsrc = e + 32 * kHelpers < e1 ? __ldg(a.ext + e + 32 * kHelpers) : 0;
+            nsrc = e + 32 * kHelpers < e1 ? __ldg(ext + e + 32 * kHelpers) : 0;
             polls = 0;
-        } else if (!keep_waiting(polls, t0, a.err, 1)) {
+        } else if (!keep_waiting(polls, t0, err, 1)) {
             return;
         }
     }
 }
 
-// the copying warp's lane: chunk c of the strip into stage c mod S once the walking warp is done with
-// chunk c - S
+// the walking warp: the fetched entries [got, end) of a chunk are there (false: given up).  first: one of them
+// per lane, looked at before; where all were there and they are at most 32, nothing is waited for.
 template <typename TX>
-__device__ void copy_chunks(const Args<TX>& a, int c0, int c1, unsigned char* stages, uint64_t* bars,
-                            const volatile int* done) {
-    const int S = a.stages;
-    const Stage L = stage_layout(a.max_width, sizeof(TX));
-    const unsigned pb = (unsigned)sizeof(TX) * kPos;
+__device__ __forceinline__ bool await_entries(int got, int end, typename Bits<TX>::U first, const unsigned char* slots,
+                                              int lane, int* err) {
+    bool ok = true;
+    if (end - got > 32 || __any_sync(0xffffffffu, first == Bits<TX>::kPending)) {
+        for (int e = got + lane; e < end; e += 32) {
+            const unsigned char* slot = slots + e % kSlots * (int)sizeof(TX);
+            long polls = 0;
+            unsigned long long t0 = 0;
+            while (ok && get<TX>(slot) == Bits<TX>::kPending) ok = keep_waiting(polls, t0, err, 1);
+        }
+        __syncwarp();
+    }
+    return ok;
+}
+
+// the copying warp's lane: chunk c of the strip's c0 .. c1 into stage (c - c0) mod S once the walking warp is done
+// with chunk c - S; issue(c, stage, barrier) announces the chunk's bytes and starts its copies
+template <typename F>
+__device__ __forceinline__ void copy_chunks(int c0, int c1, int S, int stage_bytes, unsigned char* stages, uint64_t* bars,
+                                            const volatile int* done, int* err, F issue) {
     int c = c0;
     for (; c < c1; c++) {
-        const int4 tb = __ldg(a.table + c);
         long polls = 0;
         unsigned long long t0 = 0;
         bool ok = true;
-        while (ok && *done < c - c0 - S + 1) ok = keep_waiting(polls, t0, a.err, 1);
+        while (ok && *done < c - c0 - S + 1) ok = keep_waiting(polls, t0, err, 1);
         if (!ok) break;
-        unsigned char* st = stages + ((c - c0) % S) * L.bytes;
-        uint64_t* bar = bars + (c - c0) % S;
         bulk::fence_proxy_async();  // the stage was last read through ordinary loads
-        bulk::mbar_expect_tx(bar, pb * (3u + 2u * tb.y));
-        bulk::copy(st + L.point, a.point + (size_t)c * kPos, 2u * pb, bar);
-        bulk::copy(st + L.b, a.b + (size_t)c * kPos, pb, bar);
-        if (tb.y) bulk::copy(st + L.entry, a.entry + tb.x, 2u * pb * tb.y, bar);
+        issue(c, stages + ((c - c0) % S) * stage_bytes, bars + (c - c0) % S);
     }
     // no copy may still be landing when the block exits, also where the walking warp gave up
     for (int k = c - S > c0 ? c - S : c0; k < c; k++)
@@ -231,6 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) solve_kernel(const Args<TX> a) {
     unsigned char* stages = strip_smem + kHead + operand_bytes(a.ring, sizeof(TX));
     unsigned char* ops = strip_smem + kHead;  // the ring, the slots, a zero
     unsigned char* slots = ops + a.ring * 32 * (int)sizeof(TX);
+    const Stage L = stage_layout(a.max_width, sizeof(TX));
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         ctl[0] = (int)atomicAdd(a.ticket, 1u);
@@ -244,14 +254,22 @@ __global__ void __launch_bounds__(kThreads, 1) solve_kernel(const Args<TX> a) {
     const int strip = ctl[0];
     const int c0 = __ldg(a.first + strip), c1 = __ldg(a.first + strip + 1);
     if (warp >= 2) {
-        fetch_entries<TX>(a, strip, threadIdx.x - 64, slots);
+        fetch_entries<TX>(a.x, a.ext, __ldg(a.ext_first + strip), __ldg(a.ext_first + strip + 1), threadIdx.x - 64, slots,
+                          a.err);
         return;
     }
     if (warp == 1) {
-        if (lane == 0) copy_chunks<TX>(a, c0, c1, stages, bars, ctl + 1);
+        if (lane != 0) return;
+        copy_chunks(c0, c1, a.stages, L.bytes, stages, bars, ctl + 1, a.err, [&](int c, unsigned char* st, uint64_t* bar) {
+            const int4 tb = __ldg(a.table + c);
+            const unsigned pb = (unsigned)sizeof(TX) * kPos;
+            bulk::mbar_expect_tx(bar, pb * (3u + 2u * tb.y));
+            bulk::copy(st + L.point, a.point + (size_t)c * kPos, 2u * pb, bar);
+            bulk::copy(st + L.b, a.b + (size_t)c * kPos, pb, bar);
+            if (tb.y) bulk::copy(st + L.entry, a.entry + tb.x, 2u * pb * tb.y, bar);
+        });
         return;
     }
-    const Stage L = stage_layout(a.max_width, sizeof(TX));
     constexpr int W = EM > 0 ? EM : 1;
     struct Row {
         Point<TX> p;
@@ -293,15 +311,7 @@ __global__ void __launch_bounds__(kThreads, 1) solve_kernel(const Args<TX> a) {
             nphase ^= 1u;
         }
         const int w = EM > 0 ? EM : __ldg(a.table + c0 + c).y;
-        if (end - got > 32 || __any_sync(0xffffffffu, first == B::kPending)) {
-            for (int e = got + lane; e < end; e += 32) {  // the chunk's fetched entries
-                const unsigned char* slot = slots + e % kSlots * (int)sizeof(TX);
-                long polls = 0;
-                unsigned long long t0 = 0;
-                while (ok && get<TX>(slot) == B::kPending) ok = keep_waiting(polls, t0, a.err, 1);
-            }
-            __syncwarp();
-        }
+        ok = await_entries<TX>(got, end, first, slots, lane, a.err) && ok;
 #pragma unroll
         for (int i = 0; i < kSteps; i++) {
             U res;

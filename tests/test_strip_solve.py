@@ -1,4 +1,4 @@
-"""Triangular solves pipelined over strips of rows (strip_plan.h, strip_solve.cuh).
+"""Triangular solves and ILU(0) pipelined over strips of rows (strip_plan.h, strip_solve.cuh, strip_factor.cuh).
 
 The plan is walked on the CPU with the kernel's rules, its actors in random order, and the walk's solution
 is compared with the row recurrence's bit for bit (both round each product and sum as one fused operation).
@@ -16,6 +16,8 @@ import scipy.sparse as sp
 import scipy.sparse.linalg as spla
 
 from fem_gb300 import lina, problems
+from oracle import ilu as oilu
+from oracle import port
 from tests.conftest import ROOT, gpu_available
 
 
@@ -121,6 +123,43 @@ def test_wide_levels_get_no_plan(walker, lower):
     assert walk(walker, A, lower, np.ones(n))[0] == 1
     D = sp.csr_matrix(np.ones((18, 18)) + 20 * np.eye(18))
     assert walk(walker, D, lower, np.ones(18))[0] == 1
+
+
+@pytest.mark.parametrize("name", PATTERNS)
+def test_factor_plan_walk_gives_the_factors(walker, name):
+    A = PATTERNS[name]()
+    ptr, col = A.indptr.astype(np.int32), A.indices.astype(np.int32)
+    f, info = np.full(A.nnz, np.nan), np.zeros(4, np.int32)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)  # noqa: E731
+    rc = walker.strip_factor_walk(A.shape[0], p(ptr), p(col), p(A.data), p(f), p(info))
+    assert rc in (0, 1), (rc, info)
+    if rc == 0:
+        assert np.array_equal(f, oilu.ilu0(ptr, col, A.data)), info
+    if name not in ("far", "long_rows", "elasticity"):
+        assert rc == 0
+
+
+def test_quotients_round_as_the_division(walker):
+    walker.quotient_misses.restype = C.c_long
+    assert walker.quotient_misses(C.c_long(5_000_000), C.c_uint(3)) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(not gpu_available(), reason="no CUDA device")
+@pytest.mark.parametrize("scale", [1.0, 1e-200, 1e-310])
+@pytest.mark.parametrize("name", PATTERNS)
+def test_gpu_factors_equal_restatement(name, scale):
+    """Bit-identical factors, also where quotients leave the corrections' range (scaled rows) and are zeros."""
+    A = PATTERNS[name]()
+    data = A.data.copy()
+    rows = np.repeat(np.arange(A.shape[0]), np.diff(A.indptr))
+    data[rows % 5 == 2] *= scale
+    data[(rows + 1 == A.indices) & (rows % 7 == 3)] = 0.0
+    ilu = lina.ILU(A.shape[0], A.indptr, A.indices, data)
+    ref = port.ilu0(A.indptr, A.indices, data)
+    assert np.array_equal(ilu.factor_values(), ref, equal_nan=True)
+    ilu.refactor(2.0 * data)
+    assert np.array_equal(ilu.factor_values(), port.ilu0(A.indptr, A.indices, 2.0 * data), equal_nan=True)
 
 
 @pytest.mark.gpu
