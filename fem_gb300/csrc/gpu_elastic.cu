@@ -376,18 +376,99 @@ void assemble_host(const Plan& P, const double* E, double* val, double* b) {
     }
 }
 
-// ---------------------------------------------------------------- kernels
-__global__ void assemble_values_kernel(long nnz, const int* __restrict__ cptr, const int* __restrict__ celem,
-                                       const double* __restrict__ ccoef, const double* __restrict__ E,
-                                       double* __restrict__ val) {
-    for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < nnz; q += (long)gridDim.x * blockDim.x) {
-        double v = 0.0;
-        const int c1 = cptr[q + 1];
-        for (int c = cptr[q]; c < c1; c++) {
-            const int e = celem[c];
-            v = __dadd_rn(v, __dmul_rn(e >= 0 ? E[e] : 1.0, ccoef[c]));
+// The contribution lists as the device reads them: the stored entries ordered by the length of their lists and
+// cut into slices of 32 of one length (the last of a length padded with entry -1), contribution k of a slice's
+// lane l at offset + 32 k + l.
+struct Slices {
+    std::vector<int> slice;  // per slice: offset / 32, length
+    std::vector<int> entry;  // per slice and lane: the stored entry, -1 none
+    std::vector<int> elem;
+    std::vector<double> coef;
+};
+
+bool make_slices(const Plan& P, Slices& S) {
+    const long nnz = P.ptr[P.n];
+    int most = 0;
+#pragma omp parallel for schedule(static) reduction(max : most)
+    for (long q = 0; q < nnz; q++) most = std::max(most, P.cptr[q + 1] - P.cptr[q]);
+    std::vector<long> count(most + 1, 0), at(most + 1, 0);
+    for (long q = 0; q < nnz; q++) count[P.cptr[q + 1] - P.cptr[q]]++;
+    long slots = 0, total = 0;
+    for (int c = 0; c <= most; c++) {
+        at[c] = slots;
+        const long ns = (count[c] + 31) / 32;
+        for (long k = 0; k < ns; k++) {
+            S.slice.push_back((int)(total / 32));
+            S.slice.push_back(c);
+            total += 32L * c;
         }
-        val[q] = v;
+        slots += 32 * ns;
+    }
+    if (slots > INT32_MAX || total / 32 > INT32_MAX) return false;
+    S.entry.assign(slots, -1);
+    for (long q = 0; q < nnz; q++) S.entry[at[P.cptr[q + 1] - P.cptr[q]]++] = (int)q;
+    S.elem.assign(total, -1);
+    S.coef.assign(total, 0.0);
+#pragma omp parallel for schedule(static)
+    for (long t = 0; t < slots; t++) {
+        const int q = S.entry[t];
+        if (q < 0) continue;
+        const long base = 32L * S.slice[2 * (t / 32)] + t % 32;
+        for (int c = P.cptr[q]; c < P.cptr[q + 1]; c++) {
+            S.elem[base + 32L * (c - P.cptr[q])] = P.celem[c];
+            S.coef[base + 32L * (c - P.cptr[q])] = P.ccoef[c];
+        }
+    }
+    return true;
+}
+
+struct DeviceSlices {
+    long slots = 0;
+    int *slice = nullptr, *entry = nullptr, *elem = nullptr;
+    double* coef = nullptr;
+};
+
+// h: a handle with upload(); its stream is synchronised before the host lists go out of scope
+template <typename H>
+bool upload_slices(H* h, const Plan& P, DeviceSlices& D) {
+    Slices S;
+    if (!make_slices(P, S)) return false;
+    D.slots = (long)S.entry.size();
+    return h->upload(&D.slice, S.slice.data(), S.slice.size()) && h->upload(&D.entry, S.entry.data(), S.entry.size()) &&
+           h->upload(&D.elem, S.elem.data(), S.elem.size()) && h->upload(&D.coef, S.coef.data(), S.coef.size()) &&
+           cudaStreamSynchronize(h->st) == cudaSuccess;
+}
+
+// ---------------------------------------------------------------- kernels
+// One thread per stored entry: products and sums in element order, each rounded by itself (the first sum, 0 + t,
+// is t with -0 made +0, formed without the FP64 pipe).  What bounds it is GB300's FP64 issue (one warp
+// instruction in 19 cycles per SM, whatever its active lanes) next to 12 bytes a contribution: with the entries
+// in stored order every warp ran as long as its longest list (6 of a diagonal entry, where the mean is 2.6) and
+// read lists lane by lane.  In slices of one length, 2.1M unknowns of plane elasticity, 29.4M entries: 705 us
+// before, ASSEMBLE us.
+__global__ void __launch_bounds__(kT) assemble_values_kernel(long slots, const int2* __restrict__ slice,
+                                                             const int* __restrict__ entry, const int* __restrict__ elem,
+                                                             const double* __restrict__ coef,
+                                                             const double* __restrict__ E, double* __restrict__ val) {
+    for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < slots; t += (long)gridDim.x * blockDim.x) {
+        const int2 sl = __ldg(slice + (t >> 5));
+        const int q = __ldcs(entry + t);
+        const int* ep = elem + 32L * sl.x + (t & 31);
+        const double* cp = coef + 32L * sl.x + (t & 31);
+        double v = 0.0;
+        for (int k = 0; k < sl.y; k += 2) {  // two contributions' loads together
+            const bool two = k + 1 < sl.y;
+            const int e0 = __ldcs(ep + 32 * k), e1 = two ? __ldcs(ep + 32 * (k + 1)) : -1;
+            const double c0 = __ldcs(cp + 32 * k), c1 = two ? __ldcs(cp + 32 * (k + 1)) : 0.0;
+            const double f0 = e0 >= 0 ? __ldg(E + e0) : 1.0, f1 = e1 >= 0 ? __ldg(E + e1) : 1.0;
+            const double t0 = __dmul_rn(f0, c0);
+            if (k == 0)
+                v = ((unsigned)__double2loint(t0) | ((unsigned)__double2hiint(t0) ^ 0x80000000u)) == 0 ? 0.0 : t0;
+            else
+                v = __dadd_rn(v, t0);
+            if (two) v = __dadd_rn(v, __dmul_rn(f1, c1));
+        }
+        if (q >= 0) val[q] = v;
     }
 }
 
@@ -463,9 +544,9 @@ struct lina_gpu_elastic {
     Plan plan;
     lina_gpu_amg* amg = nullptr;
     cudaStream_t st = nullptr;
-    int *d_cptr = nullptr, *d_celem = nullptr, *d_lptr = nullptr, *d_lelem = nullptr, *d_tri = nullptr,
-        *d_sdof = nullptr;
-    double *d_ccoef = nullptr, *d_lcoef = nullptr, *d_fixval = nullptr, *d_geo = nullptr, *d_target = nullptr;
+    DeviceSlices slices;
+    int *d_lptr = nullptr, *d_lelem = nullptr, *d_tri = nullptr, *d_sdof = nullptr;
+    double *d_lcoef = nullptr, *d_fixval = nullptr, *d_geo = nullptr, *d_target = nullptr;
     unsigned char* d_fixed = nullptr;
     double *d_E = nullptr, *d_val = nullptr, *d_b = nullptr, *d_u = nullptr, *d_lam = nullptr, *d_src = nullptr,
            *d_grad = nullptr, *d_loss = nullptr;
@@ -506,11 +587,16 @@ bool cuda_ok(cudaError_t e, const char* what) {
     return false;
 }
 
+void launch_values(const DeviceSlices& D, const double* coef, double* val, cudaStream_t st) {
+    if (D.slots > 0)
+        assemble_values_kernel<<<grid(D.slots), kT, 0, st>>>(D.slots, reinterpret_cast<const int2*>(D.slice), D.entry,
+                                                             D.elem, D.coef, coef, val);
+}
+
 // assemble A(E) and b on the device from d_E
 bool assemble_device(lina_gpu_elastic* h) {
     const Plan& P = h->plan;
-    const long nnz = P.ptr[P.n];
-    assemble_values_kernel<<<grid(nnz), kT, 0, h->st>>>(nnz, h->d_cptr, h->d_celem, h->d_ccoef, h->d_E, h->d_val);
+    launch_values(h->slices, h->d_E, h->d_val, h->st);
     assemble_rhs_kernel<<<grid(P.n), kT, 0, h->st>>>(P.n, h->d_lptr, h->d_lelem, h->d_lcoef, h->d_fixed, h->d_fixval,
                                                      h->d_E, h->d_b);
     return cuda_ok(cudaGetLastError(), "assembly launch");
@@ -563,8 +649,7 @@ int lina_gpu_elastic_create(const lina_gpu_elastic_problem* p, const double* you
     }
     h->ns = p->n_sensors;
     bool ok = cuda_ok(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking), "stream");
-    ok = ok && h->upload(&h->d_cptr, P.cptr.data(), P.cptr.size()) && h->upload(&h->d_celem, P.celem.data(), P.celem.size()) &&
-         h->upload(&h->d_ccoef, P.ccoef.data(), P.ccoef.size()) && h->upload(&h->d_lptr, P.lptr.data(), P.lptr.size()) &&
+    ok = ok && upload_slices(h, P, h->slices) && h->upload(&h->d_lptr, P.lptr.data(), P.lptr.size()) &&
          h->upload(&h->d_lelem, P.lelem.data(), P.lelem.size()) && h->upload(&h->d_lcoef, P.lcoef.data(), P.lcoef.size()) &&
          h->upload(&h->d_fixed, P.fixed.data(), P.fixed.size()) && h->upload(&h->d_fixval, P.fixval.data(), P.fixval.size()) &&
          h->upload(&h->d_geo, P.geo.data(), P.geo.size()) && h->upload(&h->d_tri, p->tri, 3L * P.ne) &&
@@ -700,8 +785,9 @@ int lina_gpu_elastic_destroy(lina_gpu_elastic* h) {
 struct lina_gpu_p1 {
     Plan plan;
     cudaStream_t st = nullptr;
-    int *d_cptr = nullptr, *d_celem = nullptr, *d_lptr = nullptr, *d_lelem = nullptr;
-    double *d_ccoef = nullptr, *d_lcoef = nullptr, *d_fixval = nullptr, *d_coef = nullptr, *d_val = nullptr,
+    DeviceSlices slices;
+    int *d_lptr = nullptr, *d_lelem = nullptr;
+    double *d_lcoef = nullptr, *d_fixval = nullptr, *d_coef = nullptr, *d_val = nullptr,
            *d_b = nullptr;
     unsigned char* d_fixed = nullptr;
     std::vector<void*> mem;
@@ -765,9 +851,7 @@ int lina_gpu_p1_create(const lina_gpu_p1_problem* p, lina_gpu_p1** out) {
     }
     const long nnz = P.ptr[P.n];
     bool ok = cuda_ok(cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking), "stream");
-    ok = ok && h->upload(&h->d_cptr, P.cptr.data(), P.cptr.size()) &&
-         h->upload(&h->d_celem, P.celem.data(), P.celem.size()) &&
-         h->upload(&h->d_ccoef, P.ccoef.data(), P.ccoef.size()) && h->upload(&h->d_lptr, P.lptr.data(), P.lptr.size()) &&
+    ok = ok && upload_slices(h, P, h->slices) && h->upload(&h->d_lptr, P.lptr.data(), P.lptr.size()) &&
          h->upload(&h->d_lelem, P.lelem.data(), P.lelem.size()) &&
          h->upload(&h->d_lcoef, P.lcoef.data(), P.lcoef.size()) &&
          h->upload(&h->d_fixed, P.fixed.data(), P.fixed.size()) &&
@@ -792,8 +876,7 @@ int lina_gpu_p1_assemble(lina_gpu_p1* h, const double* coef, int flags) {
             return LINA_GPU_ECUDA;
         c = h->d_coef;
     }
-    const long nnz = P.ptr[P.n];
-    assemble_values_kernel<<<grid(nnz), kT, 0, h->st>>>(nnz, h->d_cptr, h->d_celem, h->d_ccoef, c, h->d_val);
+    launch_values(h->slices, c, h->d_val, h->st);
     assemble_rhs_kernel<<<grid(P.n), kT, 0, h->st>>>(P.n, h->d_lptr, h->d_lelem, h->d_lcoef, h->d_fixed, h->d_fixval, c,
                                                      h->d_b);
     if (!cuda_ok(cudaGetLastError(), "assembly") || !cuda_ok(cudaStreamSynchronize(h->st), "assembly"))
