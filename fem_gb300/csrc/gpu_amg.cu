@@ -85,13 +85,15 @@ void set_err(const char* fmt, ...) {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 16384;     // partials per reduction value
+constexpr int kFewRows = 152 * 4 * kThreads;  // one wave of sell_kernel's R_FEW variant
 constexpr int kGridCap = 152 * 12;    // grid-stride cap: 152 SMs x 12 blocks of 256
 constexpr int kReduceGrid = 152 * 4;  // streaming reductions: half a wave, four strides per loop trip
 
 // ---------------------------------------------------------------- reductions
 // Programmatic dependent launch: kernels of the solve are launched with programmatic stream
-// serialisation.  Each kernel first waits, before any access to global memory, until the previous grid
-// has completed and its writes are visible, then lets the next kernel's blocks be scheduled: they take
+// serialisation.  Each kernel waits, before any access to what kernels write while a solve runs, until the
+// previous grid has completed and its writes are visible (what only set-up and value updates write, ended by a
+// synchronisation of the stream, may be read before), then lets the next kernel's blocks be scheduled: they take
 // the SMs this grid's finishing blocks free and wait there, so the launch gap between the many short
 // kernels of a V-cycle is hidden.  Both instructions are no-ops for a kernel launched without the
 // attribute.
@@ -250,47 +252,108 @@ __device__ __forceinline__ int sell_col(unsigned short d, int2 base) {
 
 // rowseg / act (segmented batches, else null): the system of every row and whether it is still iterating;
 // the rows of systems that have stopped are skipped (their values are not used any more)
-template <typename TV, typename TX, int MODE, bool LONG, typename TI>
-__global__ void __launch_bounds__(kThreads) sell_kernel(int npos, int nrows, const int* __restrict__ rowmap,
+enum { R_SHORT = 0, R_FEW = 1, R_LONG = 2 };
+template <typename TV, typename TX, int MODE, int ROWS, typename TI>
+__global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel(int npos, int nrows, const int* __restrict__ rowmap,
                                                         const int* __restrict__ sptr, const int2* __restrict__ sbase,
                                                         const TI* __restrict__ col, const TV* __restrict__ val,
                                                         const TX* x, TX* y, const TX* __restrict__ b,
                                                         const TX* __restrict__ dinv, TX w, const TX* z,
                                                         double* partials, unsigned* ticket, KScalars* sc,
                                                         const int* __restrict__ rowseg, const int* __restrict__ act) {
-    pdl_wait();
     double dot = 0.0;
     // grid-stride over slice positions (npos is a multiple of 32, so warps stay whole); positions
     // past the last row (natural order) or marked -1 (colour order) are padding
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npos; t += gridDim.x * blockDim.x) {
+    int t = blockIdx.x * blockDim.x + threadIdx.x;
+    // The matrix does not change while kernels run, so a thread's first row and (R_FEW, R_LONG) its first batch of
+    // eight entries are loaded before it waits for the previous kernel.
+    constexpr bool EARLY = ROWS != R_SHORT;
+    TI c[8];
+    TV v[8];
+    bool waited = !EARLY;
+    if constexpr (!EARLY) pdl_wait();
+    for (; t < npos; t += gridDim.x * blockDim.x) {
         const int i = rowmap ? rowmap[t] : t;
-        if (i < 0 || i >= nrows) continue;
-        if (rowseg && !act[rowseg[i]]) continue;
+        const bool row = i >= 0 && i < nrows;
+        if constexpr (!EARLY) {
+            if (!row) continue;
+            if (rowseg && !act[rowseg[i]]) continue;
+        }
         const int sl = t >> 5, lane = t & 31;
-        const int p0 = sptr[sl];
-        const int len = (sptr[sl + 1] - p0) >> 5;
+        int p0 = 0, len = 0;
         int2 cb = make_int2(0, 0);
-        if constexpr (sizeof(TI) == 2) cb = __ldg(sbase + sl);
+        if (!EARLY || row) {
+            p0 = sptr[sl];
+            len = (sptr[sl + 1] - p0) >> 5;
+            if constexpr (sizeof(TI) == 2) cb = __ldg(sbase + sl);
+        }
+        // entries stream through once: evict-first loads
         const TI* cp = col + p0 + lane;
         const TV* vp = val + p0 + lane;
+        auto fetch = [&](int k) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) c[u] = __ldcs(cp + 32 * (k + u));
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = __ldcs(vp + 32 * (k + u));
+        };
+        auto fetch_rest = [&](int k) {
+#pragma unroll
+            for (int u = 0; u < 7; u++)
+                if (k + u < len) c[u] = __ldcs(cp + 32 * (k + u));
+#pragma unroll
+            for (int u = 0; u < 7; u++)
+                if (k + u < len) v[u] = __ldcs(vp + 32 * (k + u));
+        };
+        if constexpr (EARLY) {
+            if (len >= 8)
+                fetch(0);
+            else if constexpr (ROWS == R_FEW)
+                fetch_rest(0);
+            if (!waited) {
+                pdl_wait();
+                waited = true;
+            }
+            if (!row || (rowseg && !act[rowseg[i]])) continue;
+        }
         TX sum = TX(0);
+        // Batches of eight entries: the gathers of x together, then the products in stored order, so every
+        // thread keeps several loads in flight.  x is read through the read-only path (no thread reads an entry
+        // of y written by another thread of the same launch, also in the in-place SOR mode, where rows of one
+        // colour do not couple).
+        //  R_LONG (dense coarse operators): software-pipelined, the indices and values of the next batch are
+        //   loaded before the products of the current one.
+        //  R_SHORT: 32 registers, so that 64 warps an SM hide the latency.
+        //  R_FEW (short rows, at most a wave of blocks): latency is what counts, so the rest of a row after its
+        //   batches is loaded together, predicated, in 64 registers.  Measured on GB300: a segmented batch whose
+        //   colour launches are such 94 ms with R_SHORT, 80 ms with R_FEW; a sweep of 2.1M rows of 14 entries
+        //   in FP64 82 us with R_SHORT, 88 us with R_FEW.
         int k = 0;
-        // Batches of eight entries: eight index loads, eight value loads, eight gathers of x, then
-        // the products in stored order, so every thread keeps several loads in flight.  LONG rows
-        // (dense coarse operators) are software-pipelined: the indices and values of the next
-        // batch are loaded before the gathers of the current one.  Short rows run predicated
-        // batches instead (fewer registers, so more threads per SM).  The matrix streams through
-        // once (evict-first loads); x is read through the read-only path (no thread reads an
-        // entry of y written by another thread of the same launch, also in the in-place SOR
-        // mode, where rows of one colour do not couple).
-        if constexpr (LONG) {
+        if constexpr (ROWS == R_FEW) {
             if (len >= 8) {
-                TI c[8];
-                TV v[8];
+                for (k = 8;; k += 8) {
+                    TX xv[8];
 #pragma unroll
-                for (int u = 0; u < 8; u++) c[u] = __ldcs(cp + 32 * u);
+                    for (int u = 0; u < 8; u++) xv[u] = __ldg(x + sell_col(c[u], cb));
+                    const bool more = (k + 8 <= len);
 #pragma unroll
-                for (int u = 0; u < 8; u++) v[u] = __ldcs(vp + 32 * u);
+                    for (int u = 0; u < 8; u++) sum += TX(v[u]) * xv[u];
+                    if (!more) break;
+                    fetch(k);
+                }
+                fetch_rest(k);
+            }
+            if (k < len) {
+                TX xv[7];
+#pragma unroll
+                for (int u = 0; u < 7; u++)
+                    if (k + u < len) xv[u] = __ldg(x + sell_col(c[u], cb));
+#pragma unroll
+                for (int u = 0; u < 7; u++)
+                    if (k + u < len) sum += TX(v[u]) * xv[u];
+                k = len;
+            }
+        } else if constexpr (ROWS == R_LONG) {
+            if (len >= 8) {
                 for (k = 8;; k += 8) {
                     TX xv[8];
 #pragma unroll
@@ -313,13 +376,8 @@ __global__ void __launch_bounds__(kThreads) sell_kernel(int npos, int nrows, con
             }
         } else {
             for (; k + 8 <= len; k += 8) {
-                TI c[8];
-                TV v[8];
                 TX xv[8];
-#pragma unroll
-                for (int u = 0; u < 8; u++) c[u] = __ldcs(cp + 32 * (k + u));
-#pragma unroll
-                for (int u = 0; u < 8; u++) v[u] = __ldcs(vp + 32 * (k + u));
+                fetch(k);
 #pragma unroll
                 for (int u = 0; u < 8; u++) xv[u] = __ldg(x + sell_col(c[u], cb));
 #pragma unroll
@@ -327,8 +385,6 @@ __global__ void __launch_bounds__(kThreads) sell_kernel(int npos, int nrows, con
             }
         }
         if (k + 4 <= len) {
-            TI c[4];
-            TV v[4];
             TX xv[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) c[u] = __ldcs(cp + 32 * (k + u));
@@ -354,6 +410,7 @@ __global__ void __launch_bounds__(kThreads) sell_kernel(int npos, int nrows, con
             dot += double(x[i]) * double(sum);
         }
     }
+    if (!waited) pdl_wait();
     if constexpr (MODE == M_DOT) block_partial(dot, partials);
 }
 
@@ -380,27 +437,34 @@ __global__ void __launch_bounds__(kThreads, 5) sellq_kernel(int n, const int* __
                                                             const float* __restrict__ dinv, float w,
                                                             const float* z, const int* __restrict__ rowseg,
                                                             const int* __restrict__ act) {
-    pdl_wait();
-    const int npos = ((n + 31) >> 5) << 5;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npos; t += gridDim.x * blockDim.x) {
-        const int i = t;
-        if (i >= n) continue;
-        if (rowseg && !act[rowseg[i]]) continue;  // a stopped system of a segmented batch
-        const int sl = t >> 5, lane = t & 31;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // a thread per row
+    const bool on = i < n;
+    // the row's first two groups, loaded before the wait for the previous kernel (see sell_kernel)
+    int ng = 0;
+    int2 cb = make_int2(0, 0);
+    const uint2* cp = col4;
+    const float4* vp = val4;
+    uint2 c[2];
+    float4 v[2];
+    if (on) {
+        const int sl = i >> 5;
         const int g0 = sptr[sl] >> 2;
-        const int ng = (sptr[sl + 1] - sptr[sl]) >> 7;  // groups of four per row
-        const int2 cb = __ldg(sbase + sl);
-        const uint2* cp = col4 + g0 + lane;
-        const float4* vp = val4 + g0 + lane;
-        float sum = 0.f;
-        int k = 0;
+        ng = (sptr[sl + 1] - sptr[sl]) >> 7;  // groups of four per row
+        cb = __ldg(sbase + sl);
+        cp += g0 + (i & 31);
+        vp += g0 + (i & 31);
         if (ng >= 2) {
-            uint2 c[2];
-            float4 v[2];
 #pragma unroll
             for (int u = 0; u < 2; u++) c[u] = __ldcs(cp + 32 * u);
 #pragma unroll
             for (int u = 0; u < 2; u++) v[u] = __ldcs(vp + 32 * u);
+        }
+    }
+    pdl_wait();
+    if (on && !(rowseg && !act[rowseg[i]])) {  // not a row of a stopped system of a segmented batch
+        float sum = 0.f;
+        int k = 0;
+        if (ng >= 2) {
             for (k = 2;; k += 2) {
                 float xv[8];
 #pragma unroll
@@ -432,12 +496,12 @@ __global__ void __launch_bounds__(kThreads, 5) sellq_kernel(int n, const int* __
             }
         }
         for (; k < ng; k++) {
-            const uint2 c = __ldcs(cp + 32 * k);
-            const float4 v = __ldcs(vp + 32 * k);
-            sum += v.x * __ldg(x + quad_col(c.x & 0xffffu, cb));
-            sum += v.y * __ldg(x + quad_col(c.x >> 16, cb));
-            sum += v.z * __ldg(x + quad_col(c.y & 0xffffu, cb));
-            sum += v.w * __ldg(x + quad_col(c.y >> 16, cb));
+            const uint2 c1 = __ldcs(cp + 32 * k);
+            const float4 v1 = __ldcs(vp + 32 * k);
+            sum += v1.x * __ldg(x + quad_col(c1.x & 0xffffu, cb));
+            sum += v1.y * __ldg(x + quad_col(c1.x >> 16, cb));
+            sum += v1.z * __ldg(x + quad_col(c1.y & 0xffffu, cb));
+            sum += v1.w * __ldg(x + quad_col(c1.y >> 16, cb));
         }
         if constexpr (MODE == M_SPMV) {
             y[i] = sum;
@@ -462,36 +526,60 @@ __global__ void __launch_bounds__(kThreads) csrv_kernel(int nrows, const int* __
                                                         const TX* __restrict__ b, const TX* __restrict__ dinv, TX w,
                                                         const TX* z, double* partials, unsigned* ticket,
                                                         KScalars* sc) {
-    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int sub = lane & (S - 1);
     const long warp_global = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long nwarps = ((long)gridDim.x * blockDim.x) >> 5;
     double dot = 0.0;
-    for (long gb = warp_global * (32 / S); gb < nrows; gb += nwarps * (32 / S)) {
+    // a group's row, and its first four strides of entries: loaded before the wait for the previous kernel the
+    // first time (see sell_kernel)
+    bool valid = false;
+    int i = 0, k = 0, e0 = 0;
+    TX di = TX(0);
+    int c[4];
+    TV v[4];
+    auto fetch = [&]() {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k + u * S < e0) c[u] = __ldcs(col + k + u * S);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (k + u * S < e0) v[u] = __ldcs(val + k + u * S);
+    };
+    auto start = [&](long gb) {
         const long g = gb + lane / S;
-        const bool valid = g < nrows;
-        int i = 0, s0 = 0, e0 = 0;
+        valid = g < nrows;
+        i = k = e0 = 0;
         if (valid) {
             i = rows ? rows[g] : (int)g;
-            s0 = ptr[i];
+            k = ptr[i] + sub;
             e0 = ptr[i + 1];
+            if constexpr (MODE == M_JACOBI || MODE == M_SOR)
+                if (sub == 0) di = dinv[i];
+        }
+        fetch();
+    };
+    bool waited = false;
+    for (long gb = warp_global * (32 / S); gb < nrows; gb += nwarps * (32 / S)) {
+        start(gb);
+        if (!waited) {
+            pdl_wait();
+            waited = true;
         }
         TX sum = TX(0);
-        int k = s0 + sub;
-        // four strides of the group at a time: independent loads in flight, products summed in order
-        for (; k + 3 * S < e0; k += 4 * S) {
-            const int c0 = __ldcs(col + k), c1 = __ldcs(col + k + S), c2 = __ldcs(col + k + 2 * S),
-                      c3 = __ldcs(col + k + 3 * S);
-            const TV v0 = __ldcs(val + k), v1 = __ldcs(val + k + S), v2 = __ldcs(val + k + 2 * S),
-                     v3 = __ldcs(val + k + 3 * S);
-            const TX x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-            sum += TX(v0) * x0;
-            sum += TX(v1) * x1;
-            sum += TX(v2) * x2;
-            sum += TX(v3) * x3;
+        // four strides of the group at a time (the last ones cut short): independent loads in flight, products
+        // summed in order
+        while (k < e0) {
+            TX xv[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k + u * S < e0) xv[u] = __ldg(x + c[u]);
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k + u * S < e0) sum += TX(v[u]) * xv[u];
+            k += 4 * S;
+            if (k < e0) fetch();
         }
-        for (; k < e0; k += S) sum += TX(__ldcs(val + k)) * __ldg(x + __ldcs(col + k));
 #pragma unroll
         for (int o = S / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, S);
         if (valid && sub == 0) {
@@ -500,7 +588,7 @@ __global__ void __launch_bounds__(kThreads) csrv_kernel(int nrows, const int* __
             } else if constexpr (MODE == M_RESID) {
                 y[i] = b[i] - sum;
             } else if constexpr (MODE == M_JACOBI || MODE == M_SOR) {
-                y[i] = x[i] + w * dinv[i] * (b[i] - sum);
+                y[i] = x[i] + w * di * (b[i] - sum);
             } else if constexpr (MODE == M_ADD) {
                 y[i] = z[i] + sum;
             } else if constexpr (MODE == M_DOT) {
@@ -509,6 +597,7 @@ __global__ void __launch_bounds__(kThreads) csrv_kernel(int nrows, const int* __
             }
         }
     }
+    if (!waited) pdl_wait();
     if constexpr (MODE == M_DOT) block_partial(dot, partials);
 }
 
@@ -520,9 +609,17 @@ template <typename TB, typename TX>
 __global__ void jacobi_first_kernel(int n, const TB* __restrict__ b, const double* __restrict__ sign,
                                     const TX* __restrict__ dinv, const double* __restrict__ isoinv, TX w,
                                     TX* __restrict__ x, TX* __restrict__ bout) {
-    pdl_wait();
     const long S = (long)gridDim.x * blockDim.x;
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    // a thread with fewer than four rows loads what does not change for its first before the wait
+    TX d0 = TX(0);
+    double s0 = 0.0;
+    const bool few = i + 3 * S >= n && i < n;
+    if (few) {
+        d0 = dinv[i];
+        s0 = isoinv ? isoinv[i] : 0.0;
+    }
+    pdl_wait();
     auto one = [&](long k, double bd, TX di, double iso) {
         if (sign) bd *= sign[k];
         const TX bi = TX(bd);
@@ -543,6 +640,10 @@ __global__ void jacobi_first_kernel(int n, const TB* __restrict__ b, const doubl
 #pragma unroll
         for (int u = 0; u < 4; u++) one(i + u * S, bb[u], di[u], iso[u]);
     }
+    if (few) {
+        one(i, double(b[i]), d0, s0);
+        i += S;
+    }
     for (; i < n; i += S) one(i, double(b[i]), dinv[i], isoinv ? isoinv[i] : 0.0);
 }
 
@@ -559,45 +660,70 @@ __global__ void init_x_kernel(int n, const TB* __restrict__ b, const double* __r
     }
 }
 
-// coarsest level: gather the block right-hand side, solve the single-nonzero rows
+// coarsest level: the single-nonzero rows, and a dense FP64 GEMV with the block inverse, one warp per block row
+// (brows: the level's rows in the block).  A block-diagonal coarsest level (rblk non-null: the block of each block
+// row, its first position boff[k] and inverse offset ioff[k]) multiplies each row by its own block only; with one
+// block the arithmetic is the same.  The right-hand side is read in place (gathering it first took a launch of
+// its own), eight entries of a row and their places together, the first eight before the wait.
 template <typename TX>
-__global__ void coarse_gather_kernel(int n, const TX* __restrict__ b, const int* __restrict__ inblock,
-                                     const int* __restrict__ blockpos, const double* __restrict__ dginv,
-                                     double* __restrict__ bblk, TX* __restrict__ x) {
-    pdl_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (inblock[i])
-            bblk[blockpos[i]] = double(b[i]);
-        else
-            x[i] = TX(double(b[i]) * dginv[i]);
-    }
-}
-
-// dense FP64 GEMV with the block inverse: one warp per block row.  A block-diagonal coarsest level
-// (rblk non-null: the block of each block row, its first position boff[k] and inverse offset ioff[k])
-// multiplies each row by its own block only; with one block the arithmetic is the same.
-template <typename TX>
-__global__ void coarse_gemv_kernel(int m, const double* __restrict__ inv, const double* __restrict__ bblk,
-                                   const int* __restrict__ brows, TX* __restrict__ x, const int* __restrict__ rblk,
-                                   const int* __restrict__ boff, const long* __restrict__ ioff) {
-    pdl_wait();
+__global__ void __launch_bounds__(kThreads) coarse_solve_kernel(int n, int m, const double* __restrict__ inv,
+                                                                const TX* __restrict__ b,
+                                                                const int* __restrict__ brows, TX* __restrict__ x,
+                                                                const int* __restrict__ rblk,
+                                                                const int* __restrict__ boff,
+                                                                const long* __restrict__ ioff,
+                                                                const int* __restrict__ inblock,
+                                                                const double* __restrict__ dginv) {
     const int lane = threadIdx.x & 31;
-    for (long r = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < m;
-         r += ((long)gridDim.x * blockDim.x) >> 5) {
+    const long id = (long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long)gridDim.x * blockDim.x;
+    long r = id >> 5;
+    const double* row = inv;
+    const int* at = brows;
+    int len = 0;
+    double a[8];
+    int p[8];
+    auto fetch = [&](int j) {
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (j + 32 * u < len) {
+                a[u] = __ldg(row + j + 32 * u);
+                p[u] = __ldg(at + j + 32 * u);
+            }
+    };
+    auto start = [&]() {
         long base = r * (long)m;
-        int m0 = 0, len = m;
+        int m0 = 0;
+        len = m;
         if (rblk) {
             const int k = rblk[r];
             m0 = boff[k];
             len = boff[k + 1] - m0;
             base = ioff[k] + (r - m0) * (long)len;
         }
-        const double* row = inv + base;
-        const double* bb = bblk + m0;
+        row = inv + base;
+        at = brows + m0;
+        fetch(lane);
+    };
+    if (r < m) start();
+    pdl_wait();
+    for (long i = id; i < n; i += threads)
+        if (!inblock[i]) x[i] = TX(double(b[i]) * dginv[i]);
+    while (r < m) {
         double s = 0.0;
-        for (int j = lane; j < len; j += 32) s += row[j] * bb[j];
+        for (int j = lane; j < len; j += 256) {
+            double v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (j + 32 * u < len) v[u] = double(b[p[u]]);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+                if (j + 32 * u < len) s += a[u] * v[u];
+            fetch(j + 256);
+        }
         s = warp_sum(s);
         if (lane == 0) x[brows[r]] = TX(s);
+        r += threads >> 5;
+        if (r < m) start();
     }
 }
 
@@ -1332,8 +1458,8 @@ __global__ void __launch_bounds__(kFuseThreads, 1) fused_step_kernel(const Fused
 // copies its block's images into shared memory with asynchronous copies issued before it waits for the
 // previous kernel, gathers b for its rows, and sweeps colour by colour from shared memory: the only
 // traffic of a colour is the new entries of x, stored into every block's copy, and a cluster barrier (a
-// block barrier where K is 1).  The pre-step's residual is summed from the images too where the natural
-// matrix has the same lane groups; restriction and prolongation read R, P and the vectors from global
+// block barrier where K is 1).  The pre-step's residual is summed from the images too, in the natural
+// matrix's lane groups; restriction and prolongation read R, P and the vectors from global
 // memory as the unstaged step does.  Rows are summed by the lane groups and in the order of csrv_kernel,
 // so results are bit-identical to the per-colour launches.
 constexpr int kStagedSmemMax = 210 * 1024;
@@ -1458,16 +1584,10 @@ __global__ void __launch_bounds__(kFuseThreads, 1) staged_step_kernel(const Fuse
     }
     if (PRE) {
         TX* r = (TX*)st.r;
-        if (st.aS == S) {  // the natural matrix sums its rows in the same lane groups: from the images
-            staged_rows<TX>(0, P, S, soff, scol, sv, xs, [&](int q, TX sum, int sub) {
-                if (sub == 0) r[srow[q]] = sb[q] - sum;
-            });
-        } else {
-            fused_rows<TX>(0, st.n, st.aS, st.aptr, st.acol, (const TX*)st.aval, LocalRead<TX>{xs, 0},
-                           [&](int i, TX sum, int sub) {
-                               if (sub == 0) r[i] = b[i] - sum;
-                           });
-        }
+        // in the lane groups of the natural matrix, from the images (a row's entries lie in its order there)
+        staged_rows<TX>(0, P, st.aS, soff, scol, sv, xs, [&](int q, TX sum, int sub) {
+            if (sub == 0) r[srow[q]] = sb[q] - sum;
+        });
         fused_sync(cl);
         TX* cb = (TX*)st.cb;
         fused_rows<TX>(0, st.nc, st.rS, st.rptr, st.rcol, (const TX*)st.rval, GlobalRead<TX>{r},
@@ -1533,6 +1653,7 @@ struct DCsr {
     std::vector<int> group_slice;   // colour c occupies slices [group_slice[c], group_slice[c+1])
     // CSR-vector layout (lanes > 0): CSR arrays and, for colour groups, the rows of each colour
     int lanes = 0;
+    int lanes64 = 0;                // lanes per row of the FP64 passes
     int* ptr = nullptr;
     int* rows = nullptr;
     std::vector<int> group_row;     // colour c: rows[group_row[c] .. group_row[c+1])
@@ -1541,21 +1662,49 @@ struct DCsr {
     int max_group_rows = 0;         // rows of the largest colour
 };
 
-// Layout choice, from sweeps of every level of the 2.1M-dof elasticity hierarchy on GB300 in every
-// layout (FP32 and FP64): one thread per row (SELL-32; long rows software-pipelined) for levels of
-// 100k rows or more; a group of lanes per row for the small coarse levels, 8 lanes from 8k rows
-// (enough rows to fill the GPU, several loads in flight per lane), wider groups below.
-int csrv_lanes_for_shape(long n, double avg) {
+// Layout choice, from sweeps of every level of elasticity (97 to 1,025 squared nodes) and Poisson hierarchies on
+// GB300 in every layout.  One thread per row (SELL-32; long rows software-pipelined) from 32,768 rows on: there
+// are enough of them, and each FP64 instruction, which costs an SM 19 cycles whatever its active lanes, does 32
+// rows' work (FP64 sweeps, one thread per row against 8 lanes per row: 34,814 rows of 8.5 entries 3.3 against
+// 6.9 us, 50,748 rows of 53 entries 9.9 against 14.8, 70,011 of 95 19.7 against 24.0, 34,046 of 113 14.9 against
+// 16.4; FP32 passes of such matrices read quads in either layout).  Below, a group of lanes per row, 8 lanes
+// from 8k rows (enough rows to fill the GPU, several loads in flight per lane), wider groups below.  A
+// colour-grouped matrix is swept colour by colour: its colours must have the rows to fill the GPU (groups: their
+// number), or, as before, 100,000 rows in all.
+int csrv_lanes_for_shape(long n, double avg, long groups) {
     if (g_layout == 1) return 0;
     if (g_layout >= 3) return 4 << (g_layout - 3);
-    if (g_layout == 0 && n >= 100000 && avg <= 256.0) return 0;
+    const bool many = groups > 0 ? n >= 100000 || (avg < 24.0 && n >= 16384 * groups) : n >= 32768;
+    if (g_layout == 0 && many && avg <= 256.0) return 0;
     if (avg < 8.0) return 4;
     if (n >= 8000) return 8;
     return avg >= 24.0 ? 16 : 8;
 }
 
-int csrv_lanes_for(const lina::Csr& c) {
-    return csrv_lanes_for_shape(c.n, c.n > 0 ? double(c.nnz()) / c.n : 0.0);
+int csrv_lanes_for(const lina::Csr& c, const std::vector<std::vector<int>>* groups) {
+    return csrv_lanes_for_shape(c.n, c.n > 0 ? double(c.nnz()) / c.n : 0.0, groups ? (long)groups->size() : 0);
+}
+
+// Lanes per row of the FP64 passes over a natural-order matrix in the lane-group layout (the arrays are the same
+// for any number of lanes).  The time in cycles is modelled as the larger of the FP64 issue (per group of rows
+// the products of one lane, log2 S sums of the butterfly and two operations of the update, 19 cycles each, over
+// 152 SMs) and three quarters of the longest row's chain (about 1,180 cycles per batch of four strides: two L2
+// round trips and four products of 64 cycles).  Sweeps on GB300, the lanes of the rule above against these:
+// 18,818 rows of 14 entries 4.4 (8 lanes) against 3.6 us (4), 23,862 rows of 92 entries 13.7 (8) against 9.7 (4),
+// 3,196 rows of 4 to 119 entries 5.9 (4) against 3.7 (16), 1,339 rows of 72 entries 3.7 (16) against 3.4 (32).
+int csrv_lanes64_for(long n, double avg, int longest) {
+    int best = 4;
+    double best_t = 0.0;
+    for (int S = 4, lg = 2; S <= 32; S *= 2, lg++) {
+        const double pipe = n * (avg + S * (lg + 2)) / 32.0 * 19.0 / 152.0;
+        const double chain = 0.75 * (1180.0 * ((longest + 4 * S - 1) / (4 * S)) + 90.0 * lg);
+        const double t = std::max(pipe, chain);
+        if (S == 4 || t < best_t) {
+            best = S;
+            best_t = t;
+        }
+    }
+    return best;
 }
 
 // Host-side SELL-32 construction; `order` lists the rows per group (colour)
@@ -1816,8 +1965,8 @@ struct DLevel {
 
 // every non-CSR launch goes through here so that the library can report how many
 // kernels it issued
-// Every kernel of this file starts with pdl_wait(), so it may be launched with programmatic stream
-// serialisation (g_pdl, default on): its blocks start while the previous kernel drains, which hides most
+// Every kernel of this file waits (pdl_wait) before it touches what another kernel of a solve writes, so it may
+// be launched with programmatic stream serialisation (g_pdl, default on): its blocks start while the previous kernel drains, which hides most
 // of the launch gap between the many short kernels of a V-cycle.
 template <typename... KA, typename... A>
 void launch(void (*k)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... a) {
@@ -1869,10 +2018,8 @@ struct lina_gpu_amg {
     int cm = 0;
     int* c_brows = nullptr;
     int* c_inblock = nullptr;
-    int* c_blockpos = nullptr;
     double* c_inv = nullptr;
     double* c_dginv = nullptr;
-    double* c_bblk = nullptr;
     int *c_rblk = nullptr, *c_boff = nullptr;  // block-diagonal coarsest level (else null)
     long* c_ioff = nullptr;
     // finest-level extras
@@ -1981,6 +2128,16 @@ struct lina_gpu_amg {
         if (count) CK(cudaMemcpyAsync(*p, src, count * sizeof(T), cudaMemcpyHostToDevice, stream));
         return 0;
     }
+    // the rule's layout: a level of a segmented batch with long rows takes that of its largest system's level
+    // (lanes_rows rows): concatenated small levels keep the lane groups their long rows need.  Short rows go by
+    // the rows of all systems together (FP32 sweeps of 296k rows of 14 entries: one thread per row 5.3 us, 8 lanes
+    // 14.1 us)
+    int rule_lanes(const lina::Csr& c, const std::vector<std::vector<int>>* groups) const {
+        const double avg = c.n > 0 ? double(c.nnz()) / c.n : 0.0;
+        const long rows = lanes_rows > 0 && avg >= 24.0 ? std::min<long>(lanes_rows, c.n) : c.n;
+        return csrv_lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0);
+    }
+
     // pos_out (optional): the stored position of every CSR entry (-1: not stored), empty for the
     // lane-group layout, whose positions are the CSR order
     int upload_csr(DCsr& d, const lina::Csr& c, const std::vector<std::vector<int>>* groups = nullptr,
@@ -2002,13 +2159,16 @@ struct lina_gpu_amg {
             set_err("matrix entry with column %d outside [0, %d)", c.col[bad], ncols);
             return LINA_GPU_EINVAL;
         }
-        // a level of a segmented batch takes the layout of its largest system's level (lanes_rows rows):
-        // concatenated small levels keep the lane groups their long rows need; an autotuned level the
-        // layout measured fastest (force_lanes)
-        d.lanes = force_lanes >= 0 ? force_lanes
-                  : lanes_rows > 0 ? csrv_lanes_for_shape(std::min<long>(lanes_rows, c.n), c.n > 0 ? double(c.nnz()) / c.n : 0.0)
-                                   : csrv_lanes_for(c);
+        // an autotuned level takes the layout measured fastest (force_lanes), any other the rule's
+        d.lanes = force_lanes >= 0 ? force_lanes : rule_lanes(c, groups);
         if (d.lanes > 0) {
+            d.lanes64 = d.lanes;
+            if (!groups && force_lanes < 0 && g_layout < 3) {
+                int longest = 0;
+#pragma omp parallel for schedule(static) reduction(max : longest)
+                for (int r = 0; r < c.n; r++) longest = std::max(longest, c.ptr[r + 1] - c.ptr[r]);
+                d.lanes64 = csrv_lanes64_for(c.n, c.n > 0 ? double(c.nnz()) / c.n : 0.0, longest);
+            }
             // CSR-vector: sanitise placeholder columns outside the operand, keep the CSR arrays
             std::vector<int> colc(c.col);
             for (size_t k = 0; k < colc.size(); k++)
@@ -2148,21 +2308,24 @@ struct lina_gpu_amg {
         const dim3 gd(grid), bd(kThreads);
         // row indices of a natural-order range start at 32 slice0; of the colour order, they are global
         const int* rseg = (mask_rows && m.rowseg) ? (rm ? m.rowseg : m.rowseg + (size_t)32 * slice0) : nullptr;
-        if (sizeof(TX) == 4 && m.col16) {
-            const int2* sb = m.sbase + slice0;
-            if (m.long_rows)
-                launch(sell_kernel<TV, TX, MODE, true, unsigned short>, gd, bd, 0, stream, npos, nrows, rm, sp, sb,
-                       (const unsigned short*)m.col16, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);
-            else
-                launch(sell_kernel<TV, TX, MODE, false, unsigned short>, gd, bd, 0, stream, npos, nrows, rm, sp, sb,
-                       (const unsigned short*)m.col16, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);
-        } else if (m.long_rows) {
-            launch(sell_kernel<TV, TX, MODE, true, int>, gd, bd, 0, stream, npos, nrows, rm, sp, (const int2*)nullptr,
-                   (const int*)m.col, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);
-        } else {
-            launch(sell_kernel<TV, TX, MODE, false, int>, gd, bd, 0, stream, npos, nrows, rm, sp, (const int2*)nullptr,
-                   (const int*)m.col, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);
-        }
+        const bool c16 = sizeof(TX) == 4 && m.col16;
+        const int2* sb = c16 ? m.sbase + slice0 : nullptr;
+#define LINA_SELL(R)                                                                                               \
+    do {                                                                                                           \
+        if (c16)                                                                                                   \
+            launch(sell_kernel<TV, TX, MODE, R, unsigned short>, gd, bd, 0, stream, npos, nrows, rm, sp, sb,       \
+                   (const unsigned short*)m.col16, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);   \
+        else                                                                                                       \
+            launch(sell_kernel<TV, TX, MODE, R, int>, gd, bd, 0, stream, npos, nrows, rm, sp, sb,                  \
+                   (const int*)m.col, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);                \
+    } while (0)
+        if (m.long_rows)
+            LINA_SELL(R_LONG);
+        else if (npos <= kFewRows)
+            LINA_SELL(R_FEW);
+        else
+            LINA_SELL(R_SHORT);
+#undef LINA_SELL
         if (MODE == M_DOT) launch(dot_finish_kernel, dim3(1), dim3(1024), 0, stream, grid, (const double*)partials, sc);
     }
 
@@ -2181,7 +2344,7 @@ struct lina_gpu_amg {
                 return;
             }
         }
-        const int S = m.lanes;
+        const int S = sizeof(TX) == 8 ? m.lanes64 : m.lanes;
         long grid = ((long)nrows * S + kThreads - 1) / kThreads;
         if (MODE == M_DOT && grid > kMaxBlocks) grid = kMaxBlocks;
         if (grid > (1L << 30)) grid = 1L << 30;
@@ -2262,12 +2425,9 @@ struct lina_gpu_amg {
     template <typename TX>
     void coarse_solve(const TX* b, TX* x) {
         const int n = lv[0].n;
-        go(coarse_gather_kernel<TX>, grid_for(n, kThreads), stream, n, b, c_inblock, c_blockpos,
-                                                                                 c_dginv, c_bblk, x);
-        if (cm > 0)
-            go(coarse_gemv_kernel<TX>, grid_for((long)cm * 32, kThreads), stream, cm, (const double*)c_inv,
-               (const double*)c_bblk, (const int*)c_brows, x, (const int*)c_rblk, (const int*)c_boff,
-               (const long*)c_ioff);
+        go(coarse_solve_kernel<TX>, grid_for(std::max((long)cm * 32, (long)n), kThreads), stream, n, cm,
+           (const double*)c_inv, b, (const int*)c_brows, x, (const int*)c_rblk, (const int*)c_boff,
+           (const long*)c_ioff, (const int*)c_inblock, (const double*)c_dginv);
     }
 
     // pre-smoothing from the zero guess (plus the isolated-row fix on the finest level)
@@ -2382,10 +2542,11 @@ struct lina_gpu_amg {
         st.nc = C.n;
         st.ncolours = L.ncolours;
         st.nu = nu;
-        st.sS = L.Acol.lanes;
-        st.aS = L.A.lanes;
-        st.rS = L.R.lanes;
-        st.pS = L.P.lanes;
+        constexpr bool f64 = sizeof(TX) == 8;
+        st.sS = f64 ? L.Acol.lanes64 : L.Acol.lanes;
+        st.aS = f64 ? L.A.lanes64 : L.A.lanes;
+        st.rS = f64 ? L.R.lanes64 : L.R.lanes;
+        st.pS = f64 ? L.P.lanes64 : L.P.lanes;
         st.sptr = L.Acol.ptr;
         st.scol = L.Acol.col;
         st.srows = L.Acol.rows;
@@ -2619,6 +2780,10 @@ struct lina_gpu_amg {
                 go(convert_kernel<double, float>, grid_for(L.n, kThreads), stream, L.n, r, L.b32);
                 coarse_solve<float>(L.b32, kz32);
             } else {
+                if (r == z) {  // in place: the solve reads all of r while it writes z
+                    cudaMemcpyAsync(L.b64, r, (size_t)L.n * sizeof(double), cudaMemcpyDeviceToDevice, stream);
+                    r = L.b64;
+                }
                 coarse_solve<double>(r, z);
             }
             return;
@@ -2901,9 +3066,7 @@ int autotune_level(lina_gpu_amg* h, const lina::HostLevel& hl, int l, const std:
     int best = -1;
     const TX w = TX(h->opt.omega);
     std::string report;
-    const int rule = h->lanes_rows > 0 ? csrv_lanes_for_shape(std::min<long>(h->lanes_rows, n),
-                                                               n > 0 ? double(hl.A.nnz()) / n : 0.0)
-                                        : csrv_lanes_for(hl.A);
+    const int rule = h->rule_lanes(hl.A, sor ? &colours : nullptr);
     float rule_ms = 0.f;
     if ((rc = h->alloc(&x, n)) || (rc = h->alloc(&y, n)) || (rc = h->upload(&b, ones.data(), ones.size())) ||
         (rc = h->upload(&dv, dinv.data(), dinv.size())))
@@ -3153,11 +3316,8 @@ int upload_hierarchy(lina_gpu_amg* h) {
     lina::CoarseSolver& cs = H.coarse;
     h->cm = (int)cs.block_rows.size();
     h->c_block_rows = cs.block_rows;
-    std::vector<int> blockpos(cs.n, 0);
-    for (int k = 0; k < h->cm; k++) blockpos[cs.block_rows[k]] = k;
     if ((rc = h->upload(&h->c_brows, cs.block_rows.data(), cs.block_rows.size()))) return rc;
     if ((rc = h->upload(&h->c_inblock, cs.in_block.data(), cs.in_block.size()))) return rc;
-    if ((rc = h->upload(&h->c_blockpos, blockpos.data(), blockpos.size()))) return rc;
     if ((rc = h->upload(&h->c_inv, cs.inv.data(), cs.inv.size()))) return rc;
     if (cs.blocks.empty()) {
         if (!cs.inverted) {  // a large block: inverted in place on the device
@@ -3190,7 +3350,6 @@ int upload_hierarchy(lina_gpu_amg* h) {
         }
     }
     if ((rc = h->upload(&h->c_dginv, cs.diag_inv.data(), cs.diag_inv.size()))) return rc;
-    if ((rc = h->alloc(&h->c_bblk, std::max(h->cm, 1)))) return rc;
     // finest extras
     const int nf = H.lv[depth - 1].A.n;
     {
@@ -3646,7 +3805,7 @@ namespace {
 
 // CSR entry -> layout position for a matrix uploaded by upload_csr (same layout choice)
 std::vector<int> layout_positions(const lina::Csr& c, const std::vector<std::vector<int>>* groups) {
-    if (csrv_lanes_for(c) > 0) {
+    if (csrv_lanes_for(c, groups) > 0) {
         std::vector<int> pos(c.nnz());
         for (long k = 0; k < c.nnz(); k++) pos[k] = (int)k;
         return pos;
