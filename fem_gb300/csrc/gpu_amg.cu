@@ -22,6 +22,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
+#include <numeric>
 #include <string>
 #include <vector>
 
@@ -1452,26 +1454,40 @@ __global__ void __launch_bounds__(kFuseThreads, 1) fused_step_kernel(const Fused
 // ------------------------------------------------------------ staged fused steps
 // A fused step whose sweeps read nothing but shared memory.  At upload the level's rows are dealt to
 // the K blocks of a cluster colour by colour (each block takes a contiguous share of every colour's
-// rows) and each block's share is packed into two fixed-size images: ints (per colour the block's first
-// local position, then its rows, their entry offsets and their columns) and values (the rows' entries,
-// then omega / a_ii; gathered again on the device whenever the level's values or omega change).  A step
-// copies its block's images into shared memory with asynchronous copies issued before it waits for the
-// previous kernel, gathers b for its rows, and sweeps colour by colour from shared memory: the only
-// traffic of a colour is the new entries of x, stored into every block's copy, and a cluster barrier (a
-// block barrier where K is 1).  The pre-step's residual is summed from the images too, in the natural
-// matrix's lane groups; restriction and prolongation read R, P and the vectors from global
-// memory as the unstaged step does.  Rows are summed by the lane groups and in the order of csrv_kernel,
-// so results are bit-identical to the per-colour launches.
+// rows, longest rows first) and each block's share is packed into two fixed-size images: ints (per colour the
+// block's first local position and log2 of the FP64 lanes per row, then its rows, their entry offsets, the blocks that
+// need their entries of x, and their columns) and values (the rows' entries, then omega / a_ii; gathered again
+// on the device whenever the level's values or omega change).  A step copies its block's images into shared
+// memory with asynchronous copies issued before it waits for the previous kernel, gathers b for its rows, and
+// sweeps colour by colour from shared memory: the only traffic of a colour is the new entries of x, stored into
+// the copies of the blocks whose rows couple to them, and a cluster barrier (a block barrier where K is 1).  The
+// pre-step's residual is summed from the images too, in the natural matrix's lane groups; restriction and
+// prolongation read R, P and the vectors from global memory as the unstaged step does.  Rows are summed by the
+// lane groups and in the order of csrv_kernel, so results are bit-identical to the per-colour launches.
+//
+// A level made of independent systems (a segmented batch) runs as several clusters in one launch, each with a
+// group of whole systems: its own rows, coarse rows and images.
+//
+// What bounds a colour: the cluster barrier, and in FP64 the SM's four FP64 units, each issuing one warp
+// instruction in 64 cycles whatever its active lanes.  So the FP64 lanes per row are chosen colour by colour
+// (stage_lanes64): a few long rows take wide groups (a shorter chain of products), many short ones narrow groups
+// (no sums over the group).  A colour of a few rows costs about 2,100 cycles: its sums 950, update and stores 490,
+// arriving at the barrier 385.  Measured on GB300, pre-steps of P1 Poisson 257 x 257 in FP64 (9,214, 3,072, 1,561
+// and 1,154 rows): 53, 50, 67 and 79 us with one number of lanes a level, every entry stored into 16 copies and a
+// colour's rows looked up after its barrier; 28, 37, 54 and 55 us now; whole solves 7.41 -> 5.56 ms.  A segmented
+// batch of 16 systems (608,657 unknowns), whose three lowest levels below the coarsest run as 6 or 7 clusters where
+// they took a launch per colour or an unstaged cluster: 80 -> 53 ms.
 constexpr int kStagedSmemMax = 210 * 1024;
 
 struct StagedPlan {
-    const int* img;    // K int images of `ints` ints
-    const void* vals;  // K value images of `nvals` values (TX)
+    const int* img;      // K int images of `ints` ints per group
+    const void* vals;    // K value images of `nvals` values (TX) per group
+    const int4* groups;  // per cluster: its rows [x, y) and coarse rows [z, w)
     int ints, nvals;
-    int pslots;               // b slots (the largest share's positions, a multiple of 4)
-    int o_row, o_off, o_col;  // sections of an int image
-    int o_dinv;               // 1/a_ii in a value image
-    int xbytes;               // the copy of x, a multiple of 16 bytes
+    int pslots;          // b slots (the largest share's positions, a multiple of 4)
+    int o_row, o_off, o_mask, o_col;  // sections of an int image (masks and columns: 16 bits each)
+    int o_dinv;          // 1/a_ii in a value image
+    int xbytes;          // the copy of x, a multiple of 16 bytes
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -1484,122 +1500,210 @@ __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// sum_k val_k x_col_k over entries [k0, k1) of the shared images by a group of S lanes, in the order of
-// csrv_kernel; the butterfly leaves the sum in every lane of the group
+// the sum over a group of S lanes, left in each of them (the order of csrv_kernel's butterfly)
 template <typename TX>
-__device__ __forceinline__ TX staged_row_sum(bool valid, int k0, int k1, int sub, int S, const int* scol,
-                                             const TX* sv, const TX* xs) {
-    TX sum = TX(0);
-    if (valid) {
-        // eight, then four strides at a time: the loads of a batch are in flight together (the sums
-        // stay in order)
-        int k = k0 + sub;
-        for (; k + 7 * S < k1; k += 8 * S) {
-            int c[8];
-            TX v[8], x[8];
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                c[j] = scol[k + j * S];
-                v[j] = sv[k + j * S];
-            }
-#pragma unroll
-            for (int j = 0; j < 8; j++) x[j] = xs[c[j]];
-#pragma unroll
-            for (int j = 0; j < 8; j++) sum += v[j] * x[j];
-        }
-        if (k + 3 * S < k1) {
-            const int c0 = scol[k], c1 = scol[k + S], c2 = scol[k + 2 * S], c3 = scol[k + 3 * S];
-            const TX v0 = sv[k], v1 = sv[k + S], v2 = sv[k + 2 * S], v3 = sv[k + 3 * S];
-            const TX x0 = xs[c0], x1 = xs[c1], x2 = xs[c2], x3 = xs[c3];
-            sum += v0 * x0;
-            sum += v1 * x1;
-            sum += v2 * x2;
-            sum += v3 * x3;
-            k += 4 * S;
-        }
-        for (; k < k1; k += S) sum += sv[k] * xs[scol[k]];
-    }
-    for (int o = S / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, S);
+__device__ __forceinline__ TX group_sum(TX sum, int S) {
+    if (S > 16) sum += __shfl_xor_sync(0xffffffffu, sum, 16, 32);
+    if (S > 8) sum += __shfl_xor_sync(0xffffffffu, sum, 8, 32);
+    if (S > 4) sum += __shfl_xor_sync(0xffffffffu, sum, 4, 32);
+    if (S > 2) sum += __shfl_xor_sync(0xffffffffu, sum, 2, 32);
+    if (S > 1) sum += __shfl_xor_sync(0xffffffffu, sum, 1, 32);
     return sum;
 }
 
-// f(q, sum, sub) for every local position q of [q0, q1), called by every lane of its group.  Consecutive
-// positions share a warp: an FP64 instruction costs the SM's FP64 pipe the same with one active lane as
-// with 32, so rows are packed into as few warps as possible.
-template <typename TX, typename F>
-__device__ __forceinline__ void staged_rows(int q0, int q1, int S, const int* soff, const int* scol, const TX* sv,
-                                            const TX* xs, F f) {
-    const int lane = threadIdx.x & 31, sub = lane & (S - 1);
-    const int warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
-    const int per_warp = 32 / S;
-    for (int qb = q0 + warp * per_warp; qb < q1; qb += nwarps * per_warp) {
-        const int q = qb + lane / S;
-        const bool valid = q < q1;
-        const TX sum = staged_row_sum<TX>(valid, valid ? soff[q] : 0, valid ? soff[q + 1] : 0, sub, S, scol, sv, xs);
-        if (valid) f(q, sum, sub);
+// A row of a staged level as one lane of its group of S holds it: what is needed besides the entries of x that
+// other rows change.  Its first four strides of entries are in registers.
+template <typename TX>
+struct StageRow {
+    bool warp_on, on;  // the warp has rows, the group has one
+    int i, k, k1, col[4];
+    unsigned mask;
+    TX v[4], wdi, b, x;
+};
+
+// the rest of a row's sum is read in batches of four strides (the last cut short), a batch's loads in flight
+// together, products in the order of csrv_kernel
+template <typename TX>
+__device__ __forceinline__ void stage_entries(StageRow<TX>& r, int S, const unsigned short* scol, const TX* sv) {
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+        if (r.k + u * S < r.k1) {
+            r.col[u] = scol[r.k + u * S];
+            r.v[u] = sv[r.k + u * S];
+        }
+}
+
+template <typename TX>
+__device__ __forceinline__ TX stage_sum(StageRow<TX>& r, int S, const unsigned short* scol, const TX* sv,
+                                        const TX* xs) {
+    TX sum = TX(0);
+    while (r.k < r.k1) {
+        TX x[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (r.k + u * S < r.k1) x[u] = xs[r.col[u]];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (r.k + u * S < r.k1) sum += r.v[u] * x[u];
+        r.k += 4 * S;
+        if (r.k < r.k1) stage_entries(r, S, scol, sv);
     }
+    return group_sum(sum, S);
+}
+
+// For every local position q of [q0, q1): v = value(q, row sum), then store(q, v, sub), each by every lane of
+// its group, the stores after all lanes of the warp have formed their values.  Consecutive positions share a
+// warp: an FP64 instruction costs the SM's FP64 pipe the same with one active lane as with 32, so rows are
+// packed into as few warps as possible.
+template <typename TX, typename V, typename F>
+__device__ __forceinline__ void staged_rows(int q0, int q1, int lg, const int* soff, const unsigned short* scol,
+                                            const TX* sv, const TX* xs, V value, F store) {
+    const int S = 1 << lg, lane = threadIdx.x & 31, sub = lane & (S - 1);
+    const int warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
+    const int per_warp = 32 >> lg;
+    for (int qb = q0 + warp * per_warp; qb < q1; qb += nwarps * per_warp) {
+        const int q = qb + (lane >> lg);
+        const bool valid = q < q1;
+        StageRow<TX> r;
+        r.k = valid ? soff[q] + sub : 0;
+        r.k1 = valid ? soff[q + 1] : 0;
+        stage_entries(r, S, scol, sv);
+        const TX sum = stage_sum(r, S, scol, sv, xs);
+        const TX v = valid ? value(q, sum) : TX(0);
+        __syncwarp();
+        if (valid) store(q, v, sub);
+    }
+}
+
+// entry i of the own copy of x and of the copies of the blocks in mask := v, the group's S lanes sharing the stores
+template <typename TX>
+__device__ __forceinline__ void store_needed(const cg::cluster_group& cl, TX* xs, int i, TX v, unsigned mask, int sub,
+                                             int S) {
+    if (sub == 0) xs[i] = v;
+    if (S >= 8) {  // a lane per block, or two
+        for (int r = sub; r < 16; r += S)
+            if (mask >> r & 1u) cl.map_shared_rank(xs, (unsigned)r)[i] = v;
+        return;
+    }
+    for (int t = 0; mask; t++, mask &= mask - 1)
+        if ((t & (S - 1)) == sub) cl.map_shared_rank(xs, (unsigned)(__ffs(mask) - 1))[i] = v;
 }
 
 template <typename TX, bool PRE>
 __global__ void __launch_bounds__(kFuseThreads, 1) staged_step_kernel(const FusedStep st, const StagedPlan sp) {
     extern __shared__ __align__(16) unsigned char staged_smem[];
     const cg::cluster_group cl = cg::this_cluster();
-    const int K = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+    const int rank = (int)cl.block_rank();
     TX* xs = reinterpret_cast<TX*>(staged_smem);
     TX* sv = reinterpret_cast<TX*>(staged_smem + sp.xbytes);
     TX* sb = sv + sp.nvals;
     int* si = reinterpret_cast<int*>(sb + sp.pslots);
     {  // the block's images (static between value refreshes): copied while the previous kernel drains
-        const char* gi = reinterpret_cast<const char*>(sp.img + (long)rank * sp.ints);
-        const char* gv = reinterpret_cast<const char*>(static_cast<const TX*>(sp.vals) + (long)rank * sp.nvals);
+        const char* gi = reinterpret_cast<const char*>(sp.img + (long)blockIdx.x * sp.ints);
+        const char* gv = reinterpret_cast<const char*>(static_cast<const TX*>(sp.vals) + (long)blockIdx.x * sp.nvals);
         const int ni = sp.ints / 4, nv = sp.nvals * (int)sizeof(TX) / 16;
         for (int j = (int)threadIdx.x; j < ni; j += blockDim.x) cp_async16(reinterpret_cast<char*>(si) + 16 * j, gi + 16 * j);
         for (int j = (int)threadIdx.x; j < nv; j += blockDim.x) cp_async16(reinterpret_cast<char*>(sv) + 16 * j, gv + 16 * j);
     }
+    const int4 grp = __ldg(sp.groups + blockIdx.x / cl.num_blocks());
+    const int r0 = grp.x, nr = grp.y - grp.x;
     pdl_wait();
     TX* xg = (TX*)st.x;
     const TX* b = (const TX*)st.b;
-    for (int j = (int)threadIdx.x; j < st.n; j += blockDim.x) xs[j] = PRE ? TX(0) : __ldcg(xg + j);
+    for (int j = (int)threadIdx.x; j < nr; j += blockDim.x) xs[j] = PRE ? TX(0) : __ldcg(xg + r0 + j);
     cp_async_wait_all();
     __syncthreads();
     const int C = st.ncolours, P = si[C];
-    const int *srow = si + sp.o_row, *soff = si + sp.o_off, *scol = si + sp.o_col;
+    const int *srow = si + sp.o_row, *soff = si + sp.o_off;
+    const unsigned short* smask = reinterpret_cast<const unsigned short*>(si + sp.o_mask);
+    const unsigned short* scol = reinterpret_cast<const unsigned short*>(si + sp.o_col);
     const TX* swdi = sv + sp.o_dinv;  // omega / a_ii
     for (int q = (int)threadIdx.x; q < P; q += blockDim.x) sb[q] = __ldg(b + srow[q]);
     fused_sync(cl);  // every copy of x is set before any remote store
-    if (!PRE) {
-        fused_rows<TX>(0, st.n, st.pS, st.pptr, st.pcol, (const TX*)st.pval, GlobalRead<TX>{(const TX*)st.e},
-                       [&](int i, TX sum, int sub) { broadcast_x(xs, i, xs[i] + sum, sub, st.pS); });
+    const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5), nwarps = (int)(blockDim.x >> 5);
+    if (!PRE) {  // x += P e on the block's rows
+        const int S = st.pS, per_warp = 32 / S, sub = lane & (S - 1);
+        for (int qb = warp * per_warp; qb < P; qb += nwarps * per_warp) {
+            const int q = qb + lane / S;
+            const bool valid = q < P;
+            const int i = valid ? srow[q] : 0;
+            const TX sum = fused_row_sum<TX>(valid, valid ? __ldg(st.pptr + i) : 0, valid ? __ldg(st.pptr + i + 1) : 0,
+                                             sub, S, st.pcol, (const TX*)st.pval, GlobalRead<TX>{(const TX*)st.e});
+            const TX v = valid ? xs[i - r0] + sum : TX(0);
+            __syncwarp();  // the group's lanes have read the entry before one of them stores it
+            if (valid) store_needed(cl, xs, i - r0, v, smask[q], sub, S);
+        }
         fused_sync(cl);
     }
-    const int S = st.sS;
+    // The sweeps.  A colour's first rows (one per lane group of the block) are loaded, but for the entries of x that
+    // other rows change, between arriving at the barrier before it and leaving it.  A warp without rows stays out
+    // of the sums: its FP64 instructions would cost the units' time all the same.
     const int steps = st.nu * C;
-    for (int step = 0; step < steps; step++) {
-        const int c = step % C;
-        staged_rows<TX>(si[c], si[c + 1], S, soff, scol, sv, xs, [&](int q, TX sum, int sub) {
-            const int i = srow[q];
-            broadcast_x(xs, i, xs[i] + swdi[q] * (sb[q] - sum), sub, S);
-        });
-        fused_sync(cl);
+    struct Head {
+        int q0, q1, lg;  // a colour's positions, log2 of its lanes per row
+    };
+    const int lg32 = 31 - __clz(st.sS);
+    auto head = [&](int c) { return Head{si[c], si[c + 1], sizeof(TX) == 8 ? si[C + 1 + c] : lg32}; };
+    auto fetch = [&](StageRow<TX>& r, const Head& h) {
+        const int first = h.q0 + warp * (32 >> h.lg), sub = lane & ((1 << h.lg) - 1), q = first + (lane >> h.lg);
+        r.warp_on = first < h.q1;
+        r.on = q < h.q1;
+        r.k = r.k1 = 0;
+        if (r.on) {
+            r.k = soff[q] + sub;
+            r.k1 = soff[q + 1];
+            r.i = srow[q] - r0;
+            r.mask = smask[q];
+            r.wdi = swdi[q];
+            r.b = sb[q];
+            r.x = xs[r.i];  // its own entry: written by this warp, a sweep ago
+        }
+        stage_entries(r, 1 << h.lg, scol, sv);
+    };
+    StageRow<TX> row;
+    Head h = {}, next = {};
+    if (steps > 0) {
+        h = head(0);
+        next = head(C > 1 ? 1 : 0);
+        fetch(row, h);
+    }
+    for (int step = 0, c = 0; step < steps; step++) {
+        if (row.warp_on) {
+            const int S = 1 << h.lg;
+            const TX sum = stage_sum(row, S, scol, sv, xs);
+            if (row.on) store_needed(cl, xs, row.i, row.x + row.wdi * (row.b - sum), row.mask, lane & (S - 1), S);
+        }
+        const int q0 = h.q0 + nwarps * (32 >> h.lg);
+        if (q0 < h.q1)  // more rows than the block has lane groups
+            staged_rows<TX>(
+                q0, h.q1, h.lg, soff, scol, sv, xs,
+                [&](int q, TX sum) { return xs[srow[q] - r0] + swdi[q] * (sb[q] - sum); },
+                [&](int q, TX v, int sub) { store_needed(cl, xs, srow[q] - r0, v, smask[q], sub, 1 << h.lg); });
+        __syncwarp();
+        cluster_arrive();
+        c = c + 1 < C ? c + 1 : 0;
+        h = next;
+        if (step + 1 < steps) fetch(row, h);
+        next = head(c + 1 < C ? c + 1 : 0);
+        cluster_wait();
     }
     if (PRE) {
         TX* r = (TX*)st.r;
         // in the lane groups of the natural matrix, from the images (a row's entries lie in its order there)
-        staged_rows<TX>(0, P, st.aS, soff, scol, sv, xs, [&](int q, TX sum, int sub) {
-            if (sub == 0) r[srow[q]] = sb[q] - sum;
-        });
+        staged_rows<TX>(
+            0, P, 31 - __clz(st.aS), soff, scol, sv, xs, [&](int q, TX sum) { return sb[q] - sum; },
+            [&](int q, TX v, int sub) {
+                if (sub == 0) r[srow[q]] = v;
+            });
         fused_sync(cl);
         TX* cb = (TX*)st.cb;
-        fused_rows<TX>(0, st.nc, st.rS, st.rptr, st.rcol, (const TX*)st.rval, GlobalRead<TX>{r},
+        fused_rows<TX>(grp.z, grp.w, st.rS, st.rptr, st.rcol, (const TX*)st.rval, GlobalRead<TX>{r},
                        [&](int i, TX sum, int sub) {
                            if (sub == 0) cb[i] = sum;
                        });
     }
-    // the sweeps ended with a barrier: every copy is final; each block writes its share
-    const int chunk = (st.n + K - 1) / K;
-    const int lo = rank * chunk, hi = min(st.n, lo + chunk);
-    for (int j = lo + (int)threadIdx.x; j < hi; j += blockDim.x) xg[j] = xs[j];
-    fused_sync(cl);  // no block leaves while another may still store into its shared memory
+    // no store into another block's memory follows the last barrier; each block writes its rows
+    for (int q = (int)threadIdx.x; q < P; q += blockDim.x) xg[srow[q]] = xs[srow[q] - r0];
 }
 
 // the value images of a staged level from its colour-grouped matrix and 1/a_ii: src >= 0 an entry,
@@ -1621,8 +1725,8 @@ __global__ void stage_gather_kernel(long n, const int* __restrict__ src, const d
             v = w * d64[-2 - s];
             f = float(w) * d32[-2 - s];
         }
-        o64[i] = v;
-        o32[i] = f;
+        if (o64) o64[i] = v;
+        if (o32) o32[i] = f;
     }
 }
 
@@ -1657,6 +1761,7 @@ struct DCsr {
     int* ptr = nullptr;
     int* rows = nullptr;
     std::vector<int> group_row;     // colour c: rows[group_row[c] .. group_row[c+1])
+    std::vector<int> group_lanes64; // colour c: FP64 lanes per row, where the level has a staged step (else lanes64)
     int* d_group_row = nullptr;     // the same offsets on the device
     int* d_head = nullptr;          // per position of rows: (row, ptr[row], ptr[row + 1], 0)
     int max_group_rows = 0;         // rows of the largest colour
@@ -1949,13 +2054,14 @@ struct DLevel {
     // cluster per group of whole systems (ngroups > 0)
     int ngroups = 0, max_group_rows = 0;
     FusedGroup* d_groups = nullptr;
-    // the staged fused step (stage_k blocks, 0: none); images as StagedPlan describes them
-    int stage_k = 0, stage_ints = 0, stage_nvals = 0, stage_pslots = 0;
-    int stage_o_row = 0, stage_o_off = 0, stage_o_col = 0, stage_o_dinv = 0;
-    int* stage_int = nullptr;
+    // the staged fused step (stage_k blocks per cluster, 0: none; stage_groups clusters); images as StagedPlan
+    // describes them, the FP64 values only where they fit a block's shared memory
+    int stage_k = 0, stage_groups = 0, stage_rows = 0;
+    StagedPlan stage = {};
     int* stage_src = nullptr;  // per value slot: the CSR entry, -2 - row for 1/a_ii, -1 padding
     double* stage_v64 = nullptr;
     float* stage_v32 = nullptr;
+    bool staged(bool f64) const { return stage_k > 0 && (f64 ? stage_v64 != nullptr : stage_v32 != nullptr); }
     double* dinv64 = nullptr;
     float* dinv32 = nullptr;
     int ncolours = 0;
@@ -2331,7 +2437,7 @@ struct lina_gpu_amg {
 
     template <typename TV, typename TX, int MODE>
     void launch_csrv_t(const DCsr& m, const TV* val, int r0, int r1, const TX* x, TX* y, const TX* b,
-                       const TX* dinv, TX w, const TX* z) {
+                       const TX* dinv, TX w, const TX* z, int lanes = 0) {
         const int nrows = r1 - r0;
         if (nrows <= 0) return;
         if constexpr (sizeof(TX) == 4 && (MODE == M_SPMV || MODE == M_RESID || MODE == M_JACOBI || MODE == M_ADD)) {
@@ -2344,7 +2450,7 @@ struct lina_gpu_amg {
                 return;
             }
         }
-        const int S = sizeof(TX) == 8 ? m.lanes64 : m.lanes;
+        const int S = lanes > 0 ? lanes : sizeof(TX) == 8 ? m.lanes64 : m.lanes;
         long grid = ((long)nrows * S + kThreads - 1) / kThreads;
         if (MODE == M_DOT && grid > kMaxBlocks) grid = kMaxBlocks;
         if (grid > (1L << 30)) grid = 1L << 30;
@@ -2354,12 +2460,21 @@ struct lina_gpu_amg {
         launch(csrv_kernel<TV, TX, SS, MODE>, dim3((int)grid), dim3(kThreads), 0, stream, nrows, rl,              \
                (const int*)m.ptr, (const int*)m.col, val, x, y, b, dinv, w, z, partials, ticket, sc);             \
         break;
+        if constexpr (sizeof(TX) == 8 && MODE == M_SOR) {  // the narrow groups of stage_lanes64
+            switch (S) {
+                LINA_CSRV_CASE(1)
+                LINA_CSRV_CASE(2)
+                default:
+                    break;
+            }
+        }
         switch (S) {
             LINA_CSRV_CASE(4)
             LINA_CSRV_CASE(8)
             LINA_CSRV_CASE(16)
+            LINA_CSRV_CASE(32)
             default:
-                LINA_CSRV_CASE(32)
+                break;
         }
 #undef LINA_CSRV_CASE
         if (MODE == M_DOT) launch(dot_finish_kernel, dim3(1), dim3(1024), 0, stream, (int)grid, (const double*)partials, sc);
@@ -2389,7 +2504,7 @@ struct lina_gpu_amg {
         if (m.lanes > 0) {
             if constexpr (sizeof(TX) == 8)
                 launch_csrv_t<double, TX, MODE>(m, m.v64, m.group_row[c], m.group_row[c + 1], x, y, b, dinv, w,
-                                                nullptr);
+                                                nullptr, m.group_lanes64.empty() ? 0 : m.group_lanes64[c]);
             else
                 launch_csrv_t<float, TX, MODE>(m, m.v32, m.group_row[c], m.group_row[c + 1], x, y, b, dinv, w,
                                                nullptr);
@@ -2519,12 +2634,13 @@ struct lina_gpu_amg {
             return g_fused_rows > 0 && g_fused_jacobi_entries > 0 && !timed && L.n <= g_fused_rows &&
                    L.A.nnz <= g_fused_jacobi_entries && 2 * copy_bytes <= kFusedSmemMax && L.A.lanes > 0 &&
                    L.R.lanes > 0 && L.P.lanes > 0;
+        if (g_fused_rows <= 0 || opt.smoother != LINA_SMOOTHER_MC_SOR || timed) return false;
+        if (L.staged(opt.precision != LINA_PREC_MIXED) && L.stage_rows <= g_fused_rows) return true;
         const bool whole = L.n <= g_fused_rows && copy_bytes <= kFusedSmemMax;
         const bool grouped = L.ngroups > 0 && L.max_group_rows <= g_fused_rows &&
                              (long)L.max_group_rows * (opt.precision == LINA_PREC_MIXED ? 4 : 8) <= kFusedSmemMax;
-        return g_fused_rows > 0 && opt.smoother == LINA_SMOOTHER_MC_SOR && !timed && (whole || grouped) &&
-               L.ncolours > 0 && L.Acol.lanes > 0 && L.Acol.d_group_row && L.Acol.d_head && L.A.lanes > 0 &&
-               L.R.lanes > 0 && L.P.lanes > 0;
+        return (whole || grouped) && L.ncolours > 0 && L.Acol.lanes > 0 && L.Acol.d_group_row && L.Acol.d_head &&
+               L.A.lanes > 0 && L.R.lanes > 0 && L.P.lanes > 0;
     }
 
     template <typename TX, bool PRE>
@@ -2576,8 +2692,7 @@ struct lina_gpu_amg {
         st.r = lvx<TX>(L, 3);
         st.cb = lvx<TX>(C, 2);
         st.w = opt.omega;
-        if (!JAC && L.stage_k > 0 && !(L.ngroups > 0 && L.n > g_fused_rows) &&
-            L.stage_k <= staged_cluster_max<TX, PRE>()) {
+        if (!JAC && L.staged(f64) && L.stage_rows <= g_fused_rows) {
             launch_staged<TX, PRE>(L, st);
             return;
         }
@@ -2606,20 +2721,12 @@ struct lina_gpu_amg {
     // the staged step of a level: one cluster of its plan's blocks (see staged_step_kernel)
     template <typename TX, bool PRE>
     void launch_staged(const DLevel& L, const FusedStep& st) {
-        StagedPlan sp;
-        sp.img = L.stage_int;
+        StagedPlan sp = L.stage;
         sp.vals = sizeof(TX) == 8 ? (const void*)L.stage_v64 : (const void*)L.stage_v32;
-        sp.ints = L.stage_ints;
-        sp.nvals = L.stage_nvals;
-        sp.pslots = L.stage_pslots;
-        sp.o_row = L.stage_o_row;
-        sp.o_off = L.stage_o_off;
-        sp.o_col = L.stage_o_col;
-        sp.o_dinv = L.stage_o_dinv;
-        sp.xbytes = (int)(((long)L.n * sizeof(TX) + 15) / 16 * 16);
+        sp.xbytes = (int)(((long)L.stage_rows * sizeof(TX) + 15) / 16 * 16);
         const int K = L.stage_k;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(K);
+        cfg.gridDim = dim3(K * L.stage_groups);
         cfg.blockDim = dim3(kFuseThreads);
         cfg.dynamicSmemBytes =
             (size_t)sp.xbytes + (size_t)(sp.nvals + sp.pslots) * sizeof(TX) + (size_t)sp.ints * sizeof(int);
@@ -3130,7 +3237,7 @@ done:
 // the value images of a staged level, from its current entries and 1/a_ii
 int stage_refresh(lina_gpu_amg* h, DLevel& L) {
     if (L.stage_k <= 0) return 0;
-    const long n = (long)L.stage_k * L.stage_nvals;
+    const long n = (long)L.stage_groups * L.stage_k * L.stage.nvals;
     go(stage_gather_kernel, grid_for(n, kThreads), h->stream, n, (const int*)L.stage_src, (const double*)L.Acol.v64,
        (const float*)L.Acol.v32, (const double*)L.dinv64, (const float*)L.dinv32, h->opt.omega, L.stage_v64,
        L.stage_v32);
@@ -3140,17 +3247,8 @@ int stage_refresh(lina_gpu_amg* h, DLevel& L) {
 
 static inline int pad4(long v) { return (int)((v + 3) / 4 * 4); }
 
-// The staged plan of a level (see staged_step_kernel) for a cluster of K blocks, the largest the GPU
-// schedules (16 on GB300; LINA_STAGED_K=1|2|4|8 asks for fewer); none where the images, with a copy of
-// x, do not fit a block's shared memory in FP64 (such levels' fused steps read the matrix from global
-// memory).  The largest cluster is the fastest: GB300's SM runs one FP64 warp instruction about every
-// 19 cycles, whatever its active lanes, so a colour of many rows is bound by the FP64 pipes of the
-// blocks that share it (P1 Poisson 257 x 257, FP64 solves: 10.3 ms with one block per level, 9.6 with
-// four, 8.7 with eight, 8.6 with sixteen).
-int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const std::vector<std::vector<int>>& groups) {
-    L.stage_k = 0;
-    const int n = L.n, C = L.ncolours, S = L.Acol.lanes;
-    if (S <= 0 || C <= 0 || (long)n * 8 > kStagedSmemMax || (int)groups.size() != C) return 0;
+// the cluster size of staged steps, and how many such clusters the GPU runs at a time
+int stage_cluster() {
     // every variant's launch attributes are set here, outside any stream capture
     int K = std::min(std::min(lina_gpu_amg::staged_cluster_max<double, true>(),
                               lina_gpu_amg::staged_cluster_max<double, false>()),
@@ -3160,66 +3258,251 @@ int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const std::vecto
         const int v = atoi(e);
         if (v == 1 || v == 2 || v == 4 || v == 8 || v == 16) K = std::min(K, v);
     }
-    auto share = [&](int c, int r, int& a, int& b) {
-        const long len = (long)groups[c].size();
-        a = (int)(len * r / K);
-        b = (int)(len * (r + 1) / K);
-    };
-    int pmax = 0;
-    long emax = 0;
-    for (int r = 0; r < K; r++) {
-        int P = 0;
-        long E = 0;
-        for (int c = 0; c < C; c++) {
-            int a, b;
-            share(c, r, a, b);
-            P += b - a;
-            for (int t = a; t < b; t++) E += A.ptr[groups[c][t] + 1] - A.ptr[groups[c][t]];
-        }
-        pmax = std::max(pmax, P);
-        emax = std::max(emax, E);
+    return K;
+}
+
+int stage_clusters_active(int K) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(K);
+    cfg.blockDim = dim3(kFuseThreads);
+    cfg.dynamicSmemBytes = kStagedSmemMax;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = K;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, staged_step_kernel<float, true>, &cfg) != cudaSuccess) n = 1;
+    cudaGetLastError();
+    return std::max(n, 1);
+}
+
+using Colours = std::vector<std::vector<int>>;
+
+// the rows of colour c in [r0, r1) that block r of K takes: [a, b) of the colour's (ascending) rows
+void stage_share(const std::vector<int>& rows, int r0, int r1, int r, int K, int& a, int& b) {
+    const long lo = std::lower_bound(rows.begin(), rows.end(), r0) - rows.begin();
+    const long len = (std::lower_bound(rows.begin(), rows.end(), r1) - rows.begin()) - lo;
+    a = (int)(lo + len * r / K);
+    b = (int)(lo + len * (r + 1) / K);
+}
+
+// the sections of the images that hold every group's shares (the largest ones')
+struct StageSizes {
+    int pmax = 0, emax = 0, rows = 0;
+    int o_row, o_off, o_mask, o_col, ints, nvals;
+    size_t bytes(int tx) const {
+        return ((size_t)rows * tx + 15) / 16 * 16 + (size_t)(nvals + pad4(pmax)) * tx + (size_t)ints * 4;
     }
-    const int o_row = pad4(C + 1), o_off = o_row + pad4(pmax), o_col = o_off + pad4(pmax + 1);
-    const long ints = (long)o_col + pad4(emax);
-    const long nvals = (long)pad4(emax) + pad4(pmax);
-    const long bytes = ((long)n * 8 + 15) / 16 * 16 + (nvals + pad4(pmax)) * 8 + ints * 4;
-    if (bytes > kStagedSmemMax) return 0;
-    std::vector<int> img((size_t)K * ints, 0), src((size_t)K * nvals, -1);
-    for (int r = 0; r < K; r++) {
-        int* I = img.data() + (size_t)r * ints;
-        int* V = src.data() + (size_t)r * nvals;
-        int q = 0, e = 0;
+};
+
+StageSizes stage_sizes(const lina::Csr& A, const Colours& colours, const std::vector<int4>& groups, int K) {
+    StageSizes z;
+    for (const int4& g : groups) {
+        z.rows = std::max(z.rows, g.y - g.x);
+        for (int r = 0; r < K; r++) {
+            long P = 0, E = 0;
+            for (const auto& rows : colours) {
+                int a, b;
+                stage_share(rows, g.x, g.y, r, K, a, b);
+                P += b - a;
+                for (int t = a; t < b; t++) E += A.ptr[rows[t] + 1] - A.ptr[rows[t]];
+            }
+            z.pmax = std::max<long>(z.pmax, P);
+            z.emax = (int)std::max<long>(z.emax, std::min<long>(E, INT_MAX / 16));
+        }
+    }
+    z.o_row = pad4(2 * (long)colours.size() + 1);
+    z.o_off = z.o_row + pad4(z.pmax);
+    z.o_mask = z.o_off + pad4(z.pmax + 1);
+    z.o_col = z.o_mask + pad4((z.pmax + 1) / 2);
+    z.ints = z.o_col + pad4((z.emax + 1) / 2);
+    z.nvals = pad4(z.emax) + pad4(z.pmax);
+    return z;
+}
+
+// Groups of whole systems of a segmented level for clusters of K blocks: contiguous, the most entries of a group
+// as few as the number of groups allows; as many groups as the GPU runs clusters at a time, or two or three times
+// as many where the shares do not fit.  Empty where some system is too large.
+std::vector<int4> stage_segments(const lina::Csr& A, const Colours& colours, const std::vector<int>& off,
+                                 const std::vector<int>& coff, int K, int tx) {
+    const int S = (int)off.size() - 1;
+    std::vector<long> w(S);
+    for (int i = 0; i < S; i++) w[i] = (long)A.ptr[off[i + 1]] - A.ptr[off[i]];
+    const int active = stage_clusters_active(K);
+    for (int waves = 1; waves <= 3; waves++) {
+        const int G = std::min(S, waves * active);
+        long lo = *std::max_element(w.begin(), w.end()), hi = std::accumulate(w.begin(), w.end(), 0L);
+        auto cut = [&](long cap) {
+            std::vector<int4> g;
+            for (int i = 0; i < S;) {
+                long sum = w[i];
+                int j = i + 1;
+                while (j < S && sum + w[j] <= cap) sum += w[j++];
+                g.push_back(make_int4(off[i], off[j], coff[i], coff[j]));
+                i = j;
+            }
+            return g;
+        };
+        while (lo < hi) {
+            const long mid = (lo + hi) / 2;
+            if ((int)cut(mid).size() <= G)
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        std::vector<int4> g = cut(lo);
+        const StageSizes z = stage_sizes(A, colours, g, K);
+        if (z.rows <= std::min(g_fused_rows, 65535) && z.bytes(tx) <= (size_t)kStagedSmemMax) return g;
+        if (G == S) break;
+    }
+    return {};
+}
+
+// FP64 lanes per row of a colour whose largest block's share has rows of these lengths (descending): the number
+// with the shortest time, in cycles, of the longest warp (64 a product and 60 per batch of four, 115 a sum of the
+// butterfly with its shuffles, 190 for the update) or of the SM's four FP64 units (64 an operation, shared by the
+// block's warps).
+int stage_lanes64(const std::vector<int>& len) {
+    int best = 4;
+    long best_t = LONG_MAX;
+    for (int S = 1, lg = 0; S <= 32; S *= 2, lg++) {
+        const size_t per = 32 / S;
+        long total = 0, longest = 0;
+        for (size_t q = 0; q < len.size(); q += per) {
+            const long products = (len[q] + S - 1) / S;
+            total += products + lg + 2;
+            longest = std::max(longest, 64 * products + 60 * ((products + 3) / 4) + 115 * lg + 190);
+        }
+        const long t = std::max(64 * ((total + 3) / 4), longest);
+        if (t < best_t) {
+            best = S;
+            best_t = t;
+        }
+    }
+    return best;
+}
+
+// The staged plan of a level (see staged_step_kernel): clusters of K blocks, the largest the GPU schedules (16 on
+// GB300; LINA_STAGED_K=1|2|4|8 asks for fewer), one for the level or one per group of a segmented batch; none where
+// the images, with a copy of x, do not fit a block's shared memory in FP32 (such levels' fused steps read the
+// matrix from global memory), and FP32 values only where they do not fit in FP64.  The largest cluster is the
+// fastest: a colour of many rows is bound by the FP64 units of the blocks that share it (P1 Poisson 257 x
+// 257, FP64 solves: 10.3 ms with one block per level, 9.6 with four, 8.7 with eight, 8.6 with sixteen).
+int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& colours, const std::vector<int4>& groups,
+                int K) {
+    L.stage_k = 0;
+    const int n = L.n, C = L.ncolours, S = L.Acol.lanes;
+    if (S <= 0 || C <= 0 || (int)colours.size() != C || groups.empty() || K > 16) return 0;
+    for (const int4& g : groups)
+        if (g.y - g.x > 65535 || (size_t)(g.y - g.x) * 4 > (size_t)kStagedSmemMax) return 0;
+    const StageSizes z = stage_sizes(A, colours, groups, K);
+    if (z.bytes(4) > (size_t)kStagedSmemMax) return 0;
+    const bool f64 = z.bytes(8) <= (size_t)kStagedSmemMax;
+    // the FP64 lanes of every colour, from its largest share
+    std::vector<int> lanes64(C, L.Acol.lanes64);
+    std::vector<int> len;
+    if (f64)
         for (int c = 0; c < C; c++) {
-            I[c] = q;
-            int a, b;
-            share(c, r, a, b);
-            for (int t = a; t < b; t++, q++) {
-                const int i = groups[c][t];
-                I[o_row + q] = i;
-                I[o_off + q] = e;
-                V[pad4(emax) + q] = -2 - i;
-                for (int k = A.ptr[i]; k < A.ptr[i + 1]; k++, e++) {
-                    I[o_col + e] = (A.col[k] >= 0 && A.col[k] < n) ? A.col[k] : 0;  // placeholders hold 0.0
-                    V[e] = k;
+            std::vector<int> most;
+            long most_e = -1;
+            for (const int4& g : groups)
+                for (int r = 0; r < K; r++) {
+                    int a, b;
+                    stage_share(colours[c], g.x, g.y, r, K, a, b);
+                    len.clear();
+                    long e = 0;
+                    for (int t = a; t < b; t++) {
+                        len.push_back(A.ptr[colours[c][t] + 1] - A.ptr[colours[c][t]]);
+                        e += len.back();
+                    }
+                    if (e > most_e) {
+                        most_e = e;
+                        most = len;
+                    }
+                }
+            std::sort(most.begin(), most.end(), std::greater<int>());
+            lanes64[c] = stage_lanes64(most);
+        }
+    const size_t blocks = groups.size() * K;
+    std::vector<int> img(blocks * z.ints, 0), src(blocks * z.nvals, -1);
+    std::vector<unsigned char> owner(n, 0);
+    std::vector<unsigned short> need(n, 0);
+    int bad = 0;
+#pragma omp parallel for schedule(dynamic, 1) reduction(| : bad)
+    for (size_t gi = 0; gi < groups.size(); gi++) {
+        const int4 g = groups[gi];
+        for (int r = 0; r < K; r++)
+            for (int c = 0; c < C; c++) {
+                int a, b;
+                stage_share(colours[c], g.x, g.y, r, K, a, b);
+                for (int t = a; t < b; t++) owner[colours[c][t]] = (unsigned char)r;
+            }
+        for (int i = g.x; i < g.y; i++)
+            for (int k = A.ptr[i]; k < A.ptr[i + 1]; k++) {
+                const int j = A.col[k];
+                if (j >= g.x && j < g.y)
+                    need[j] |= (unsigned short)(1u << owner[i]);
+                else if (A.val[k] != 0.0)
+                    bad = 1;  // a row that couples to another group
+            }
+        for (int r = 0; r < K; r++) {
+            int* I = img.data() + (gi * K + r) * z.ints;
+            int* V = src.data() + (gi * K + r) * z.nvals;
+            unsigned short* mask = reinterpret_cast<unsigned short*>(I + z.o_mask);
+            unsigned short* col = reinterpret_cast<unsigned short*>(I + z.o_col);
+            int q = 0, e = 0;
+            for (int c = 0; c < C; c++) {
+                I[c] = q;
+                I[C + 1 + c] = 31 - __builtin_clz((unsigned)lanes64[c]);
+                int a, b;
+                stage_share(colours[c], g.x, g.y, r, K, a, b);
+                std::vector<int> rows(colours[c].begin() + a, colours[c].begin() + b);
+                std::stable_sort(rows.begin(), rows.end(),
+                                 [&](int i, int j) { return A.ptr[i + 1] - A.ptr[i] > A.ptr[j + 1] - A.ptr[j]; });
+                for (int i : rows) {
+                    I[z.o_row + q] = i;
+                    I[z.o_off + q] = e;
+                    mask[q] = (unsigned short)(need[i] & ~(1u << r));
+                    V[pad4(z.emax) + q] = -2 - i;
+                    for (int k = A.ptr[i]; k < A.ptr[i + 1]; k++, e++) {
+                        // placeholders outside the group hold 0.0
+                        col[e] = (unsigned short)(A.col[k] >= g.x && A.col[k] < g.y ? A.col[k] - g.x : 0);
+                        V[e] = k;
+                    }
+                    q++;
                 }
             }
+            I[C] = q;
+            I[z.o_off + q] = e;
         }
-        I[C] = q;
-        I[o_off + q] = e;
     }
+    if (bad) return 0;
     int rc;
-    if ((rc = h->upload(&L.stage_int, img.data(), img.size()))) return rc;
+    int* d_img = nullptr;
+    int4* d_groups = nullptr;
+    if ((rc = h->upload(&d_img, img.data(), img.size()))) return rc;
+    if ((rc = h->upload(&d_groups, groups.data(), groups.size()))) return rc;
     if ((rc = h->upload(&L.stage_src, src.data(), src.size()))) return rc;
-    if ((rc = h->alloc(&L.stage_v64, src.size()))) return rc;
+    if (f64 && (rc = h->alloc(&L.stage_v64, src.size()))) return rc;
     if ((rc = h->alloc(&L.stage_v32, src.size()))) return rc;
     L.stage_k = K;
-    L.stage_ints = (int)ints;
-    L.stage_nvals = (int)nvals;
-    L.stage_pslots = pad4(pmax);
-    L.stage_o_row = o_row;
-    L.stage_o_off = o_off;
-    L.stage_o_col = o_col;
-    L.stage_o_dinv = pad4(emax);
+    L.stage_groups = (int)groups.size();
+    L.stage_rows = z.rows;
+    L.stage = StagedPlan{};
+    L.stage.img = d_img;
+    L.stage.groups = d_groups;
+    L.stage.ints = z.ints;
+    L.stage.nvals = z.nvals;
+    L.stage.pslots = pad4(z.pmax);
+    L.stage.o_row = z.o_row;
+    L.stage.o_off = z.o_off;
+    L.stage.o_mask = z.o_mask;
+    L.stage.o_col = z.o_col;
+    L.stage.o_dinv = pad4(z.emax);
+    if (f64) L.Acol.group_lanes64 = lanes64;
     if ((rc = stage_refresh(h, L))) return rc;
     // the host images must outlive the asynchronous uploads
     return cudaStreamSynchronize(h->stream) == cudaSuccess ? 0 : LINA_GPU_ECUDA;
@@ -3235,22 +3518,35 @@ int upload_hierarchy(lina_gpu_amg* h) {
         DLevel& L = h->lv[l];
         L.n = hl.A.n;
         h->lanes_rows = h->seg_max_rows.empty() ? 0 : h->seg_max_rows[l];
+        std::vector<int> colour;
+        Colours colours;
+        if (l > 0) {
+            L.ncolours = lina::greedy_colouring(hl.A, colour);
+            colours.assign(L.ncolours, std::vector<int>());
+            for (int i = 0; i < L.n; i++) colours[colour[i]].push_back(i);
+        }
+        // the clusters of the level's staged multicolour-SOR step: one, or one per group of a batch's systems
+        std::vector<int4> stage_groups;
+        // (the finest level's sweeps are launched colour by colour)
+        const bool inner = l > 0 && l < depth - 1;
+        const int stage_k = inner ? stage_cluster() : 0;
+        const bool segmented = !h->seg_off.empty();
+        if (inner && segmented && h->opt.smoother == LINA_SMOOTHER_MC_SOR && g_fused_rows > 0)
+            stage_groups = stage_segments(hl.A, colours, h->seg_off[l], h->seg_off[l - 1], stage_k,
+                                          h->opt.precision == LINA_PREC_MIXED ? 4 : 8);
+        else if (inner && !segmented)
+            stage_groups.push_back(make_int4(0, L.n, 0, hl.R.n));
+        const bool seg_staged = segmented && !stage_groups.empty();
         // layout autotuning of the levels below the finest (their choice is kept for re-uploads)
         // (levels of more than 50M entries, and the finest level, keep the rule: one thread per row, and
         // their candidate uploads would cost seconds.  Measured on the 96-system segmented batch: its
         // levels of 100M and 153M entries time fastest with one thread per row, as the rule chooses, and
-        // tuning them doubled the batch's creation time, 9 s to 18 s)
-        if (h->autotune && l > 0 && l < depth - 1 && hl.A.n >= 2000 && hl.A.nnz() <= 50000000L) {
+        // tuning them doubled the batch's creation time, 9 s to 18 s; a level with a staged step needs none)
+        if (h->autotune && l > 0 && l < depth - 1 && hl.A.n >= 2000 && hl.A.nnz() <= 50000000L && !seg_staged) {
             if ((int)h->tuned_lanes.size() != depth) h->tuned_lanes.assign(depth, -1);
             if (h->tuned_lanes[l] < 0) {
-                std::vector<int> colour;
-                std::vector<std::vector<int>> cgroups;
-                if (h->opt.smoother == LINA_SMOOTHER_MC_SOR) {
-                    const int nc = lina::greedy_colouring(hl.A, colour);
-                    cgroups.assign(nc, std::vector<int>());
-                    for (int i = 0; i < L.n; i++) cgroups[colour[i]].push_back(i);
-                }
                 int best = -1;
+                const Colours& cgroups = h->opt.smoother == LINA_SMOOTHER_MC_SOR ? colours : Colours();
                 rc = h->opt.precision == LINA_PREC_MIXED ? autotune_level<float>(h, hl, l, cgroups, &best)
                                                          : autotune_level<double>(h, hl, l, cgroups, &best);
                 if (rc) return rc;
@@ -3258,6 +3554,12 @@ int upload_hierarchy(lina_gpu_amg* h) {
             }
         }
         h->force_lanes = ((int)h->tuned_lanes.size() == depth) ? h->tuned_lanes[l] : -1;
+        // a staged step of a batch reads its matrices in lane groups, whatever their rows
+        auto in_groups = [&](const lina::Csr& c, const Colours* g) {
+            const int rule = h->rule_lanes(c, g);
+            return !seg_staged ? -1 : rule > 0 ? rule : c.n > 0 && c.nnz() < 8 * (long)c.n ? 4 : 8;
+        };
+        if (seg_staged) h->force_lanes = in_groups(hl.A, nullptr);
         std::vector<int> posA, posQ, posC;
         if ((rc = h->upload_csr(L.A, hl.A, nullptr, h->keep_maps ? &posA : nullptr, h->keep_maps ? &posQ : nullptr)))
             return rc;
@@ -3268,17 +3570,14 @@ int upload_hierarchy(lina_gpu_amg* h) {
         if ((rc = h->upload(&L.dinv32, dinv32.data(), dinv32.size()))) return rc;
         if (l > 0) {
             const int tuned = h->force_lanes;  // the autotuned layout is A's (and its colour-grouped copy's)
-            h->force_lanes = -1;
+            h->force_lanes = in_groups(hl.P, nullptr);
             if ((rc = h->upload_csr(L.P, hl.P))) return rc;
+            h->force_lanes = in_groups(hl.R, nullptr);
             if ((rc = h->upload_csr(L.R, hl.R))) return rc;
             h->force_lanes = tuned;
-            std::vector<int> colour;
-            L.ncolours = lina::greedy_colouring(hl.A, colour);
-            std::vector<std::vector<int>> groups(L.ncolours);
-            for (int i = 0; i < L.n; i++) groups[colour[i]].push_back(i);
-            if ((rc = h->upload_csr(L.Acol, hl.A, &groups, h->keep_maps ? &posC : nullptr))) return rc;
-            if ((rc = build_stage(h, L, hl.A, groups))) return rc;
-            if (!h->seg_off.empty() && (rc = build_fused_groups(h, l, hl, groups))) return rc;
+            if ((rc = h->upload_csr(L.Acol, hl.A, &colours, h->keep_maps ? &posC : nullptr))) return rc;
+            if ((rc = build_stage(h, L, hl.A, colours, stage_groups, stage_k))) return rc;
+            if (segmented && (rc = build_fused_groups(h, l, hl, colours))) return rc;
         }
         if (h->keep_maps) {  // in-place value updates of later recomputes
             if ((int)h->rmaps.size() != depth) h->rmaps.assign(depth, lina_gpu_amg::LevelMaps());
