@@ -1938,19 +1938,16 @@ struct DCsr {
 // 16.4; FP32 passes of such matrices read quads in either layout).  Below, a group of lanes per row, 8 lanes
 // from 8k rows (enough rows to fill the GPU, several loads in flight per lane), wider groups below.  A
 // colour-grouped matrix is swept colour by colour: its colours must have the rows to fill the GPU (groups: their
-// number), or, as before, 100,000 rows in all.
-int csrv_lanes_for_shape(long n, double avg, long groups) {
+// number), or, as before, 100,000 rows in all.  lean: the lane groups' CSR arrays, which hold no padding, up to
+// 100,000 rows (handles with a device-memory limit).
+int csrv_lanes_for_shape(long n, double avg, long groups, bool lean) {
     if (g_layout == 1) return 0;
     if (g_layout >= 3) return 4 << (g_layout - 3);
-    const bool many = groups > 0 ? n >= 100000 || (avg < 24.0 && n >= 16384 * groups) : n >= 32768;
+    const bool many = n >= 100000 || (!lean && (groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768));
     if (g_layout == 0 && many && avg <= 256.0) return 0;
     if (avg < 8.0) return 4;
     if (n >= 8000) return 8;
     return avg >= 24.0 ? 16 : 8;
-}
-
-int csrv_lanes_for(const lina::Csr& c, const std::vector<std::vector<int>>* groups) {
-    return csrv_lanes_for_shape(c.n, c.n > 0 ? double(c.nnz()) / c.n : 0.0, groups ? (long)groups->size() : 0);
 }
 
 // Lanes per row of the FP64 passes over a natural-order matrix in the lane-group layout (the arrays are the same
@@ -2347,6 +2344,7 @@ struct lina_gpu_amg {
     double* hscal = nullptr;  // device scalar for normalisation
     cudaStream_t stream = nullptr;
     long dev_bytes = 0;
+    bool lean = g_mem_limit > 0;  // a device-memory limit at creation: no layout that costs memory for speed
     std::vector<void*> allocations;
     // CUDA graph of one PCG iteration inside a device-side while loop
     cudaGraphExec_t gexec = nullptr;
@@ -2406,8 +2404,8 @@ struct lina_gpu_amg {
     // 14.1 us)
     int rule_lanes(const lina::Csr& c, const std::vector<std::vector<int>>* groups) const {
         const double avg = c.n > 0 ? double(c.nnz()) / c.n : 0.0;
-        const long rows = lanes_rows > 0 && avg >= 24.0 ? std::min<long>(lanes_rows, c.n) : c.n;
-        return csrv_lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0);
+        const long rows = lanes_rows > 0 && (avg >= 24.0 || lean) ? std::min<long>(lanes_rows, c.n) : c.n;
+        return csrv_lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean);
     }
 
     // pos_out (optional): the stored position of every CSR entry (-1: not stored), empty for the
@@ -3596,7 +3594,7 @@ int stage_lanes64(const std::vector<int>& len) {
 // the images, with a copy of x, do not fit a block's shared memory in FP32 (such levels' fused steps read the
 // matrix from global memory), and FP32 values only where they do not fit in FP64.  The largest cluster is the
 // fastest: a colour of many rows is bound by the FP64 units of the blocks that share it (P1 Poisson 257 x
-// 257, FP64 solves: 10.3 ms with one block per level, 9.6 with four, 8.7 with eight, 8.6 with sixteen).
+// 257, twelve FP64 steps of levels 1-4: 948 us with two blocks, 735 with four, 604 with eight, 513 with sixteen).
 int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& colours, const std::vector<int4>& groups,
                 int K) {
     L.stage_k = 0;
@@ -3607,6 +3605,7 @@ int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& c
     const StageSizes z = stage_sizes(A, colours, groups, K);
     if (z.bytes(4) > (size_t)kStagedSmemMax) return 0;
     const bool f64 = z.bytes(8) <= (size_t)kStagedSmemMax;
+    if (h->lean && !f64) return 0;
     // the FP64 lanes of every colour, from its largest share
     std::vector<int> lanes64(C, L.Acol.lanes64);
     std::vector<int> len;
@@ -3737,7 +3736,7 @@ int upload_hierarchy(lina_gpu_amg* h) {
         const bool inner = l > 0 && l < depth - 1;
         const int stage_k = inner ? stage_cluster() : 0;
         const bool segmented = !h->seg_off.empty();
-        if (inner && segmented && h->opt.smoother == LINA_SMOOTHER_MC_SOR && g_fused_rows > 0)
+        if (inner && segmented && !h->lean && h->opt.smoother == LINA_SMOOTHER_MC_SOR && g_fused_rows > 0)
             stage_groups = stage_segments(hl.A, colours, h->seg_off[l], h->seg_off[l - 1], stage_k,
                                           h->opt.precision == LINA_PREC_MIXED ? 4 : 8);
         else if (inner && !segmented)
@@ -4308,9 +4307,9 @@ int lina_gpu_amg_recompute(lina_gpu_amg* h, int n, const int* rowptr, const int*
 
 namespace {
 
-// CSR entry -> layout position for a matrix uploaded by upload_csr (same layout choice)
-std::vector<int> layout_positions(const lina::Csr& c, const std::vector<std::vector<int>>* groups) {
-    if (csrv_lanes_for(c, groups) > 0) {
+// CSR entry -> layout position for a matrix uploaded by upload_csr with so many lanes per row
+std::vector<int> layout_positions(const lina::Csr& c, const std::vector<std::vector<int>>* groups, int lanes) {
+    if (lanes > 0) {
         std::vector<int> pos(c.nnz());
         for (long k = 0; k < c.nnz(); k++) pos[k] = (int)k;
         return pos;
@@ -4323,7 +4322,7 @@ int build_update_maps(lina_gpu_amg* h) {
     const lina::HostLevel& F = h->host.lv[f];
     const lina::Csr& A = F.A;
     int rc;
-    std::vector<int> posA = layout_positions(A, nullptr);
+    std::vector<int> posA = layout_positions(A, nullptr, h->lv[f].A.lanes);
     if ((rc = h->upload(&h->upd_posA, posA.data(), posA.size()))) return rc;
     if (h->lv[f].A.q_val) {
         QuadHost Q;
@@ -4338,7 +4337,7 @@ int build_update_maps(lina_gpu_amg* h) {
         const int nc = lina::greedy_colouring(A, colour);
         std::vector<std::vector<int>> groups(nc);
         for (int i = 0; i < A.n; i++) groups[colour[i]].push_back(i);
-        std::vector<int> posC = layout_positions(A, &groups);
+        std::vector<int> posC = layout_positions(A, &groups, h->lv[f].Acol.lanes);
         if ((rc = h->upload(&h->upd_posAcol, posC.data(), posC.size()))) return rc;
     }
     std::vector<int> diagpos(A.n, -1);
