@@ -579,7 +579,7 @@ def run_damage(args, rank, world, local):
     peak, peak_kind = measured_peaks()
     achieved = by / (ms_apply / 1e3) / 1e9
     out["roofline"] = {"bound": "hbm", "kernel": f"FP32 ILU(0) application (forward + backward triangular solve, "
-                                                 f"{nlev} levels each way; latency-bound: one block barrier per level)",
+                                                 f"{nlev} levels each way; latency-bound: a chain of steps)",
                        "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                        "peak_kind": peak_kind, "traffic": None, "bytes_per_launch": by,
                        "avg_launch_us": ms_apply * 1e3}
