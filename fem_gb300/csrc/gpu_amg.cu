@@ -29,6 +29,7 @@
 
 #include "amg_host.h"
 #include "gpu_ops.h"
+#include "layout_rules.h"
 #include "lina_gpu.h"
 
 namespace lina {
@@ -1972,26 +1973,6 @@ struct DCsr {
     int max_group_rows = 0;         // rows of the largest colour
 };
 
-// Layout choice, from sweeps of every level of elasticity (97 to 1,025 squared nodes) and Poisson hierarchies on
-// GB300 in every layout.  One thread per row (SELL-32; long rows software-pipelined) from 32,768 rows on: there
-// are enough of them, and each FP64 instruction, which costs an SM 19 cycles whatever its active lanes, does 32
-// rows' work (FP64 sweeps, one thread per row against 8 lanes per row: 34,814 rows of 8.5 entries 3.3 against
-// 6.9 us, 50,748 rows of 53 entries 9.9 against 14.8, 70,011 of 95 19.7 against 24.0, 34,046 of 113 14.9 against
-// 16.4; FP32 passes of such matrices read quads in either layout).  Below, a group of lanes per row, 8 lanes
-// from 8k rows (enough rows to fill the GPU, several loads in flight per lane), wider groups below.  A
-// colour-grouped matrix is swept colour by colour: its colours must have the rows to fill the GPU (groups: their
-// number), or, as before, 100,000 rows in all.  lean: the lane groups' CSR arrays, which hold no padding, up to
-// 100,000 rows (handles with a device-memory limit).
-int csrv_lanes_for_shape(long n, double avg, long groups, bool lean) {
-    if (g_layout == 1) return 0;
-    if (g_layout >= 3) return 4 << (g_layout - 3);
-    const bool many = n >= 100000 || (!lean && (groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768));
-    if (g_layout == 0 && many && avg <= 256.0) return 0;
-    if (avg < 8.0) return 4;
-    if (n >= 8000) return 8;
-    return avg >= 24.0 ? 16 : 8;
-}
-
 // Lanes per row of the FP64 passes over a natural-order matrix in the lane-group layout (the arrays are the same
 // for any number of lanes).  The time in cycles is modelled as the larger of the FP64 issue (per group of rows
 // the products of one lane, log2 S sums of the butterfly and two operations of the update, 19 cycles each, over
@@ -2447,7 +2428,7 @@ struct lina_gpu_amg {
     int rule_lanes(const lina::Csr& c, const std::vector<std::vector<int>>* groups) const {
         const double avg = c.n > 0 ? double(c.nnz()) / c.n : 0.0;
         const long rows = lanes_rows > 0 && (avg >= 24.0 || lean) ? std::min<long>(lanes_rows, c.n) : c.n;
-        return csrv_lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean);
+        return layout::lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean, g_layout);
     }
 
     // pos_out (optional): the stored position of every CSR entry (-1: not stored), empty for the
@@ -2876,12 +2857,12 @@ struct lina_gpu_amg {
                    L.A.nnz <= g_fused_jacobi_entries && 2 * copy_bytes <= kFusedSmemMax && L.A.lanes > 0 &&
                    L.R.lanes > 0 && L.P.lanes > 0;
         if (g_fused_rows <= 0 || opt.smoother != LINA_SMOOTHER_MC_SOR || timed) return false;
+        if (!layout::fused_layouts(L.Acol.lanes, L.A.lanes, L.R.lanes, L.P.lanes)) return false;
         if (L.staged(opt.precision != LINA_PREC_MIXED) && L.stage_rows <= g_fused_rows) return true;
         const bool whole = L.n <= g_fused_rows && copy_bytes <= kFusedSmemMax;
         const bool grouped = L.ngroups > 0 && L.max_group_rows <= g_fused_rows &&
                              (long)L.max_group_rows * (opt.precision == LINA_PREC_MIXED ? 4 : 8) <= kFusedSmemMax;
-        return (whole || grouped) && L.ncolours > 0 && L.Acol.lanes > 0 && L.Acol.d_group_row && L.Acol.d_head &&
-               L.A.lanes > 0 && L.R.lanes > 0 && L.P.lanes > 0;
+        return (whole || grouped) && L.ncolours > 0 && L.Acol.d_group_row && L.Acol.d_head;
     }
 
     template <typename TX, bool PRE>
@@ -3640,8 +3621,9 @@ int stage_lanes64(const std::vector<int>& len) {
 int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& colours, const std::vector<int4>& groups,
                 int K) {
     L.stage_k = 0;
-    const int n = L.n, C = L.ncolours, S = L.Acol.lanes;
-    if (S <= 0 || C <= 0 || (int)colours.size() != C || groups.empty() || K > 16) return 0;
+    const int n = L.n, C = L.ncolours;
+    if (!layout::fused_layouts(L.Acol.lanes, L.A.lanes, L.R.lanes, L.P.lanes)) return 0;
+    if (C <= 0 || (int)colours.size() != C || groups.empty() || K > 16) return 0;
     for (const int4& g : groups)
         if (g.y - g.x > 65535 || (size_t)(g.y - g.x) * 4 > (size_t)kStagedSmemMax) return 0;
     const StageSizes z = stage_sizes(A, colours, groups, K);

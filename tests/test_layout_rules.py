@@ -1,0 +1,71 @@
+"""Which layout a matrix takes and which steps a level's layouts allow (layout_rules.h, gpu_amg.cu).
+
+The rules are host code, tested without a GPU; on the GPU, levels at the edges of the rules give the same
+V-cycles, bit for bit, whichever step they take.
+"""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+from fem_gb300 import lina
+from tests.conftest import ROOT, gpu_available
+
+gpu = pytest.mark.skipif(not gpu_available(), reason="no CUDA device")
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    out = str(tmp_path_factory.mktemp("rules") / "layout_rules.so")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "fem_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "c", "layout_rules_driver.cpp"), "-o", out], check=True)
+    lib = C.CDLL(out)
+    lib.rule_lanes.argtypes = [C.c_long, C.c_double, C.c_long, C.c_int, C.c_int]
+    return lib
+
+
+def test_fused_steps_need_lane_groups_everywhere(rules):
+    """A three-coloured level of 33,000 rows of three entries: its colours keep lane groups where its natural-order
+    matrix and its prolongation take one thread per row, so no fused step may read them in lane groups."""
+    acol, a, p, r = (rules.rule_lanes(*s, 0, 0) for s in ((33000, 3.0, 3), (33000, 3.0, 0), (33000, 1.5, 0), (11000, 3.0, 0)))
+    assert acol > 0 and a == 0 and p == 0 and r > 0
+    assert not rules.rule_fused(acol, a, r, p)
+    for k in range(16):
+        lanes = [8 * (k >> i & 1) for i in range(4)]
+        assert bool(rules.rule_fused(*lanes)) == (k == 15)
+
+
+def ring(n):
+    """Periodic second differences with a shift."""
+    e = np.ones(n)
+    A = sp.diags([2.1 * e, -e[:-1], -e[:-1], -1.0, -1.0], [0, 1, -1, n - 1, 1 - n], format="csr")
+    A.sort_indices()
+    return A
+
+
+@gpu
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [lina.PREC_FP64, lina.PREC_MIXED])
+def test_ring_level_above_32768_rows(precision):
+    """An odd ring's inner level of about 33,300 rows and three colours with the largest documented row limit: V-cycles
+    equal those of one launch per colour."""
+    A = ring(66603)
+    n = A.shape[0]
+    r = np.random.default_rng(4).uniform(-1, 1, n)
+    z = []
+    for rows in (49152, 0):
+        lina.set_fused_rows(rows)
+        lina.set_sell_quads(0)
+        try:
+            a = lina.AMG(n, A.indptr, A.indices, A.data, depth=4, coarsening=lina.STANDARD,
+                         smoother=lina.SMOOTHER_MC_SOR, omega=1.0, precision=precision)
+            z.append(a.vcycle(r))
+        finally:
+            lina.set_fused_rows(lina.FUSED_ROWS_DEFAULT)
+            lina.set_sell_quads(1)
+    inner = a.sizes()[-2]
+    assert inner > 32768 and a.colours(len(a.sizes()) - 2).max() == 2
+    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
