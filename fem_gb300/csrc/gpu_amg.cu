@@ -2324,6 +2324,7 @@ struct lina_gpu_amg {
     std::vector<long> seg_max_rows;
     std::vector<std::vector<int>> seg_off;  // per level, the first row of each system (and the end)
     long lanes_rows = 0;
+    long fused_limit = 0;  // while a level is uploaded: its matrices of at most so many rows are read by fused steps
     // layout autotuning: on for this hierarchy, the lanes per row forced on the next uploads (-1: the
     // rule), and per level the choice made (-1: not tuned), kept for later re-uploads (recompute)
     bool autotune = false;
@@ -2428,7 +2429,7 @@ struct lina_gpu_amg {
     int rule_lanes(const lina::Csr& c, const std::vector<std::vector<int>>* groups) const {
         const double avg = c.n > 0 ? double(c.nnz()) / c.n : 0.0;
         const long rows = lanes_rows > 0 && (avg >= 24.0 || lean) ? std::min<long>(lanes_rows, c.n) : c.n;
-        return layout::lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean, g_layout);
+        return layout::lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean, fused_limit, g_layout);
     }
 
     // pos_out (optional): the stored position of every CSR entry (-1: not stored), empty for the
@@ -3747,6 +3748,8 @@ int upload_hierarchy(lina_gpu_amg* h) {
         DLevel& L = h->lv[l];
         L.n = hl.A.n;
         h->lanes_rows = h->seg_max_rows.empty() ? 0 : h->seg_max_rows[l];
+        const bool steps = l > 0 && l < depth - 1 && (h->opt.smoother == LINA_SMOOTHER_MC_SOR || g_fused_jacobi_entries > 0);
+        h->fused_limit = steps ? g_fused_rows : 0;
         std::vector<int> colour;
         Colours colours;
         if (l > 0) {
@@ -3840,6 +3843,7 @@ int upload_hierarchy(lina_gpu_amg* h) {
         if ((rc = h->alloc(&L.r32, L.n))) return rc;
     }
     h->lanes_rows = 0;
+    h->fused_limit = 0;
     // coarsest block
     lina::CoarseSolver& cs = H.coarse;
     h->cm = (int)cs.block_rows.size();

@@ -13,12 +13,14 @@ namespace layout {
 // from 8k rows (enough rows to fill the GPU, several loads in flight per lane), wider groups below.  A
 // colour-grouped matrix is swept colour by colour: its colours must have the rows to fill the GPU (groups: their
 // number), or, as before, 100,000 rows in all.  lean: the lane groups' CSR arrays, which hold no padding, up to
-// 100,000 rows (handles with a device-memory limit).  asked: the layout of lina_gpu_set_layout.
+// 100,000 rows (handles with a device-memory limit).  fused_rows: matrices of at most so many rows are read by fused
+// steps, which need lane groups (0: none are).  asked: the layout of lina_gpu_set_layout.
 // Returns the lanes per row, 0 for one thread per row.
-inline int lanes_for_shape(long n, double avg, long groups, bool lean, int asked) {
+inline int lanes_for_shape(long n, double avg, long groups, bool lean, long fused_rows, int asked) {
     if (asked == 1) return 0;
     if (asked >= 3) return 4 << (asked - 3);
-    const bool many = n >= 100000 || (!lean && (groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768));
+    const bool many = n >= 100000 || (!lean && n > fused_rows &&
+                                      (groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768));
     if (asked == 0 && many && avg <= 256.0) return 0;
     if (avg < 8.0) return 4;
     if (n >= 8000) return 8;

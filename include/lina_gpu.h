@@ -430,7 +430,9 @@ int lina_gpu_set_layout(int layout);
    (pre: x = 0, the sweeps, the residual and the restriction; post: the prolongation and the sweeps)
    as one launch of a thread-block cluster, with cluster barriers between the colours, instead of one
    launch per colour and step; the results are bit-identical.  0 turns this off.  Takes effect for
-   solves issued afterwards (a hierarchy's captured solve graph keeps the choice it was captured with). */
+   solves issued afterwards (a hierarchy's captured solve graph keeps the choice it was captured with).
+   Levels of more than 32,767 rows are stored as these steps read them (lane groups) in hierarchies created
+   with a multicolour-SOR smoother while the limit admits them, in others they keep separate launches. */
 int lina_gpu_set_fused_rows(int max_rows);
 /* damped Jacobi: levels of at most max_entries stored entries (and the rows above) run each V-cycle step
    as one cluster launch, two copies of x in shared memory (default 0 = never: measured slower than the

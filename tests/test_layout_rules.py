@@ -23,19 +23,29 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "fem_gb300", "csrc"),
                     os.path.join(ROOT, "tests", "c", "layout_rules_driver.cpp"), "-o", out], check=True)
     lib = C.CDLL(out)
-    lib.rule_lanes.argtypes = [C.c_long, C.c_double, C.c_long, C.c_int, C.c_int]
+    lib.rule_lanes.argtypes = [C.c_long, C.c_double, C.c_long, C.c_int, C.c_long, C.c_int]
     return lib
 
 
 def test_fused_steps_need_lane_groups_everywhere(rules):
     """A three-coloured level of 33,000 rows of three entries: its colours keep lane groups where its natural-order
     matrix and its prolongation take one thread per row, so no fused step may read them in lane groups."""
-    acol, a, p, r = (rules.rule_lanes(*s, 0, 0) for s in ((33000, 3.0, 3), (33000, 3.0, 0), (33000, 1.5, 0), (11000, 3.0, 0)))
+    acol, a, p, r = (rules.rule_lanes(*s, 0, 24576, 0) for s in ((33000, 3.0, 3), (33000, 3.0, 0), (33000, 1.5, 0), (11000, 3.0, 0)))
     assert acol > 0 and a == 0 and p == 0 and r > 0
     assert not rules.rule_fused(acol, a, r, p)
     for k in range(16):
         lanes = [8 * (k >> i & 1) for i in range(4)]
         assert bool(rules.rule_fused(*lanes)) == (k == 15)
+
+
+def test_levels_within_the_row_limit_keep_lane_groups(rules):
+    """Every level that lina_gpu_set_fused_rows admits is laid out for the fused step, up to 100,000 rows."""
+    for limit in (24576, 32768, 33000, 49152, 99999):
+        for n in (1000, 24576, 32767, 32768, 33000, 49152, 99999):
+            if n <= limit:
+                lanes = [rules.rule_lanes(n, avg, g, 0, limit, 0) for avg, g in ((3.0, 3), (14.0, 2), (3.0, 0), (60.0, 0))]
+                assert min(lanes) > 0, (n, limit)
+        assert rules.rule_lanes(limit + 1, 14.0, 0, 0, limit, 0) == (0 if limit + 1 >= 32768 else 8)
 
 
 def ring(n):
@@ -50,22 +60,26 @@ def ring(n):
 @pytest.mark.gpu
 @pytest.mark.parametrize("precision", [lina.PREC_FP64, lina.PREC_MIXED])
 def test_ring_level_above_32768_rows(precision):
-    """An odd ring's inner level of about 33,300 rows and three colours with the largest documented row limit: V-cycles
-    equal those of one launch per colour."""
+    """An odd ring's inner level of about 33,300 rows and three colours with the largest documented row limit: in FP32
+    its V-cycle step is fused (fewer launches), and V-cycles equal those of one launch per colour."""
     A = ring(66603)
     n = A.shape[0]
     r = np.random.default_rng(4).uniform(-1, 1, n)
-    z = []
-    for rows in (49152, 0):
-        lina.set_fused_rows(rows)
-        lina.set_sell_quads(0)
-        try:
-            a = lina.AMG(n, A.indptr, A.indices, A.data, depth=4, coarsening=lina.STANDARD,
-                         smoother=lina.SMOOTHER_MC_SOR, omega=1.0, precision=precision)
+    z, launches = [], []
+    lina.set_sell_quads(0)  # one order of summation in the separate FP32 launches
+    lina.set_fused_rows(49152)
+    try:
+        a = lina.AMG(n, A.indptr, A.indices, A.data, depth=4, coarsening=lina.STANDARD, smoother=lina.SMOOTHER_MC_SOR,
+                     omega=1.0, precision=precision)
+        for rows in (49152, lina.FUSED_ROWS_DEFAULT, 0):
+            lina.set_fused_rows(rows)
+            before = lina.launches()
             z.append(a.vcycle(r))
-        finally:
-            lina.set_fused_rows(lina.FUSED_ROWS_DEFAULT)
-            lina.set_sell_quads(1)
-    inner = a.sizes()[-2]
-    assert inner > 32768 and a.colours(len(a.sizes()) - 2).max() == 2
-    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1])
+            launches.append(lina.launches() - before)
+    finally:
+        lina.set_fused_rows(lina.FUSED_ROWS_DEFAULT)
+        lina.set_sell_quads(1)
+    inner = len(a.sizes()) - 2
+    assert a.level_size(inner) > 32768 and a.colours(inner).max() == 2
+    assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1]) and np.array_equal(z[0], z[2])
+    assert launches[1] < launches[2] and (launches[0] < launches[1]) == (precision == lina.PREC_MIXED)
