@@ -3589,30 +3589,6 @@ std::vector<int4> stage_segments(const lina::Csr& A, const Colours& colours, con
     return {};
 }
 
-// FP64 lanes per row of a colour whose largest block's share has rows of these lengths (descending): the number
-// with the shortest time, in cycles, of the longest warp (64 a product and 60 per batch of four, 115 a sum of the
-// butterfly with its shuffles, 190 for the update) or of the SM's four FP64 units (64 an operation, shared by the
-// block's warps).
-int stage_lanes64(const std::vector<int>& len) {
-    int best = 4;
-    long best_t = LONG_MAX;
-    for (int S = 1, lg = 0; S <= 32; S *= 2, lg++) {
-        const size_t per = 32 / S;
-        long total = 0, longest = 0;
-        for (size_t q = 0; q < len.size(); q += per) {
-            const long products = (len[q] + S - 1) / S;
-            total += products + lg + 2;
-            longest = std::max(longest, 64 * products + 60 * ((products + 3) / 4) + 115 * lg + 190);
-        }
-        const long t = std::max(64 * ((total + 3) / 4), longest);
-        if (t < best_t) {
-            best = S;
-            best_t = t;
-        }
-    }
-    return best;
-}
-
 // The staged plan of a level (see staged_step_kernel): clusters of K blocks, the largest the GPU schedules (16 on
 // GB300; LINA_STAGED_K=1|2|4|8 asks for fewer), one for the level or one per group of a segmented batch; none where
 // the images, with a copy of x, do not fit a block's shared memory in FP32 (such levels' fused steps read the
@@ -3654,7 +3630,7 @@ int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& c
                     }
                 }
             std::sort(most.begin(), most.end(), std::greater<int>());
-            lanes64[c] = stage_lanes64(most);
+            lanes64[c] = layout::stage_lanes64(most, L.Acol.lanes64, g_layout);
         }
     const size_t blocks = groups.size() * K;
     std::vector<int> img(blocks * z.ints, 0), src(blocks * z.nvals, -1);
@@ -3763,7 +3739,8 @@ int upload_hierarchy(lina_gpu_amg* h) {
         const bool inner = l > 0 && l < depth - 1;
         const int stage_k = inner ? stage_cluster() : 0;
         const bool segmented = !h->seg_off.empty();
-        if (inner && segmented && !h->lean && h->opt.smoother == LINA_SMOOTHER_MC_SOR && g_fused_rows > 0)
+        if (inner && segmented && !h->lean && h->opt.smoother == LINA_SMOOTHER_MC_SOR && g_fused_rows > 0 &&
+            layout::groups_allowed(g_layout))
             stage_groups = stage_segments(hl.A, colours, h->seg_off[l], h->seg_off[l - 1], stage_k,
                                           h->opt.precision == LINA_PREC_MIXED ? 4 : 8);
         else if (inner && !segmented)

@@ -2,6 +2,11 @@
 // which kernels its layouts allow.
 #pragma once
 
+#include <algorithm>
+#include <climits>
+#include <cstddef>
+#include <vector>
+
 namespace layout {
 
 // Layout choice, from sweeps of every level of elasticity (97 to 1,025 squared nodes) and Poisson hierarchies on
@@ -31,5 +36,33 @@ inline int lanes_for_shape(long n, double avg, long groups, bool lean, long fuse
 // natural-order copy of A, R and P follow rules of their own, so one of them can have lane groups (lanes > 0)
 // where another, one thread per row, has neither lanes nor row pointers.
 inline bool fused_layouts(int acol, int a, int r, int p) { return acol > 0 && a > 0 && r > 0 && p > 0; }
+
+// A batch's staged steps lay their levels out in lane groups; a layout of one thread per row that was asked for wins.
+inline bool groups_allowed(int asked) { return asked != 1; }
+
+// FP64 lanes per row of a colour whose largest block's share has rows of these lengths (descending): the number
+// with the shortest time, in cycles, of the longest warp (64 a product and 60 per batch of four, 115 a sum of the
+// butterfly with its shuffles, 190 for the update) or of the SM's four FP64 units (64 an operation, shared by the
+// block's warps).  lanes: the layout's, which a layout asked for with its lanes keeps.
+inline int stage_lanes64(const std::vector<int>& len, int lanes, int asked) {
+    if (asked >= 3) return lanes;
+    int best = 4;
+    long best_t = LONG_MAX;
+    for (int S = 1, lg = 0; S <= 32; S *= 2, lg++) {
+        const size_t per = 32 / S;
+        long total = 0, longest = 0;
+        for (size_t q = 0; q < len.size(); q += per) {
+            const long products = (len[q] + S - 1) / S;
+            total += products + lg + 2;
+            longest = std::max(longest, 64 * products + 60 * ((products + 3) / 4) + 115 * lg + 190);
+        }
+        const long t = std::max(64 * ((total + 3) / 4), longest);
+        if (t < best_t) {
+            best = S;
+            best_t = t;
+        }
+    }
+    return best;
+}
 
 }  // namespace layout

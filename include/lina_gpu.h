@@ -423,7 +423,8 @@ int lina_gpu_device_count(void);
 int lina_gpu_set_device(int device);   /* select the GPU for hierarchies created afterwards */
 /* storage layout of matrices uploaded afterwards: 0 automatic (SELL-32 thread-per-row for levels of
    100k rows or more, CSR with a lane group per row otherwise), 1 SELL-32 always, 2 CSR lane groups
-   always (group size chosen from the mean row length), 3..6 CSR lane groups of 4, 8, 16 or 32 lanes */
+   always (group size chosen from the mean row length), 3..6 CSR lane groups of 4, 8, 16 or 32 lanes (also in
+   the colours of staged multicolour-SOR steps, which otherwise choose their FP64 lanes colour by colour) */
 int lina_gpu_set_layout(int layout);
 /* interior levels of at most max_rows rows (default 24576; a block's copy of x allows up to 49152
    rows in FP32 and 24576 in FP64) run each multicolour-SOR V-cycle step

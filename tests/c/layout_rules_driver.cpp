@@ -6,3 +6,9 @@ extern "C" int rule_lanes(long n, double avg, long groups, int lean, long fused_
 }
 
 extern "C" int rule_fused(int acol, int a, int r, int p) { return layout::fused_layouts(acol, a, r, p) ? 1 : 0; }
+
+extern "C" int rule_stage_lanes(const int* len, int count, int lanes, int asked) {
+    return layout::stage_lanes64(std::vector<int>(len, len + count), lanes, asked);
+}
+
+extern "C" int rule_groups_allowed(int asked) { return layout::groups_allowed(asked) ? 1 : 0; }

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 import scipy.sparse as sp
 
-from fem_gb300 import lina
+from fem_gb300 import lina, problems
 from tests.conftest import ROOT, gpu_available
 
 gpu = pytest.mark.skipif(not gpu_available(), reason="no CUDA device")
@@ -46,6 +46,18 @@ def test_levels_within_the_row_limit_keep_lane_groups(rules):
                 lanes = [rules.rule_lanes(n, avg, g, 0, limit, 0) for avg, g in ((3.0, 3), (14.0, 2), (3.0, 0), (60.0, 0))]
                 assert min(lanes) > 0, (n, limit)
         assert rules.rule_lanes(limit + 1, 14.0, 0, 0, limit, 0) == (0 if limit + 1 >= 32768 else 8)
+
+
+def test_layouts_asked_for_win(rules):
+    """lina_gpu_set_layout(3..6) fixes the lanes of the staged colours as well, 1 keeps a batch's levels out of lane
+    groups; 0 and 2 leave both to the rules."""
+    few, many = np.array([300, 280, 4], np.int32), np.full(4000, 7, np.int32)
+    lanes = lambda v, n, asked: rules.rule_stage_lanes(v.ctypes.data_as(C.c_void_p), len(v), n, asked)  # noqa: E731
+    for asked in (3, 4, 5, 6):
+        assert lanes(few, 4 << (asked - 3), asked) == lanes(many, 4 << (asked - 3), asked) == 4 << (asked - 3)
+    for asked in (0, 2):
+        assert lanes(few, 8, asked) == 32 and lanes(many, 8, asked) == 1
+    assert [rules.rule_groups_allowed(k) for k in range(7)] == [1, 0, 1, 1, 1, 1, 1]
 
 
 def ring(n):
@@ -83,3 +95,28 @@ def test_ring_level_above_32768_rows(precision):
     assert a.level_size(inner) > 32768 and a.colours(inner).max() == 2
     assert np.isfinite(z[0]).all() and np.array_equal(z[0], z[1]) and np.array_equal(z[0], z[2])
     assert launches[1] < launches[2] and (launches[0] < launches[1]) == (precision == lina.PREC_MIXED)
+
+
+@gpu
+@pytest.mark.gpu
+def test_one_thread_per_row_asked_for_in_a_batch():
+    """Under lina_gpu_set_layout(1) a segmented batch has no lane groups, hence no fused steps: it issues the launches
+    it issues with fused steps off, and solves alike."""
+    systems = [problems.batch_system("elasticity" if i % 2 else "poisson", 600 + 100 * i, seed=i + 1) for i in range(4)]
+    amgs = [lina.AMG.from_system(s, depth=1 + problems.batch_depth(s.n), coarsening=lina.STANDARD,
+                                 smoother=lina.SMOOTHER_MC_SOR, omega=1.0, precision=lina.PREC_MIXED, matrix_tol=0.3)
+            for s in systems]
+    out = []
+    for layout, rows in ((1, lina.FUSED_ROWS_DEFAULT), (1, 0), (0, lina.FUSED_ROWS_DEFAULT)):
+        lina.set_layout(layout)
+        lina.set_fused_rows(rows)
+        try:
+            batch = lina.SegmentedBatch(amgs)
+            before = lina.launches()
+            x, infos = batch.solve([s.b for s in systems], tol=1e-8, max_iter=1000, host_loop=True)
+            out.append((x, [i.iterations for i in infos], lina.launches() - before))
+        finally:
+            lina.set_layout(0)
+            lina.set_fused_rows(lina.FUSED_ROWS_DEFAULT)
+    assert out[0][1] == out[1][1] and out[0][2] == out[1][2] > out[2][2]
+    assert all(np.array_equal(a, b) for a, b in zip(out[0][0], out[1][0]))
