@@ -1973,28 +1973,6 @@ struct DCsr {
     int max_group_rows = 0;         // rows of the largest colour
 };
 
-// Lanes per row of the FP64 passes over a natural-order matrix in the lane-group layout (the arrays are the same
-// for any number of lanes).  The time in cycles is modelled as the larger of the FP64 issue (per group of rows
-// the products of one lane, log2 S sums of the butterfly and two operations of the update, 19 cycles each, over
-// 152 SMs) and three quarters of the longest row's chain (about 1,180 cycles per batch of four strides: two L2
-// round trips and four products of 64 cycles).  Sweeps on GB300, the lanes of the rule above against these:
-// 18,818 rows of 14 entries 4.4 (8 lanes) against 3.6 us (4), 23,862 rows of 92 entries 13.7 (8) against 9.7 (4),
-// 3,196 rows of 4 to 119 entries 5.9 (4) against 3.7 (16), 1,339 rows of 72 entries 3.7 (16) against 3.4 (32).
-int csrv_lanes64_for(long n, double avg, int longest) {
-    int best = 4;
-    double best_t = 0.0;
-    for (int S = 4, lg = 2; S <= 32; S *= 2, lg++) {
-        const double pipe = n * (avg + S * (lg + 2)) / 32.0 * 19.0 / 152.0;
-        const double chain = 0.75 * (1180.0 * ((longest + 4 * S - 1) / (4 * S)) + 90.0 * lg);
-        const double t = std::max(pipe, chain);
-        if (S == 4 || t < best_t) {
-            best = S;
-            best_t = t;
-        }
-    }
-    return best;
-}
-
 // Host-side SELL-32 construction; `order` lists the rows per group (colour)
 // and each group starts on a slice boundary.  Without groups the natural row
 // order is used.
@@ -2429,7 +2407,7 @@ struct lina_gpu_amg {
     int rule_lanes(const lina::Csr& c, const std::vector<std::vector<int>>* groups) const {
         const double avg = c.n > 0 ? double(c.nnz()) / c.n : 0.0;
         const long rows = lanes_rows > 0 && (avg >= 24.0 || lean) ? std::min<long>(lanes_rows, c.n) : c.n;
-        return layout::lanes_for_shape(rows, avg, groups ? (long)groups->size() : 0, lean, fused_limit, g_layout);
+        return layout::lanes_for(rows, c.n, c.ptr.data(), groups ? (long)groups->size() : 0, lean, fused_limit, g_layout);
     }
 
     // pos_out (optional): the stored position of every CSR entry (-1: not stored), empty for the
@@ -2457,12 +2435,8 @@ struct lina_gpu_amg {
         d.lanes = force_lanes >= 0 ? force_lanes : rule_lanes(c, groups);
         if (d.lanes > 0) {
             d.lanes64 = d.lanes;
-            if (!groups && force_lanes < 0 && g_layout < 3) {
-                int longest = 0;
-#pragma omp parallel for schedule(static) reduction(max : longest)
-                for (int r = 0; r < c.n; r++) longest = std::max(longest, c.ptr[r + 1] - c.ptr[r]);
-                d.lanes64 = csrv_lanes64_for(c.n, c.n > 0 ? double(c.nnz()) / c.n : 0.0, longest);
-            }
+            if (!groups && force_lanes < 0 && g_layout < 3)
+                d.lanes64 = layout::lanes64_for(layout::row_counts(c.n, c.ptr.data()), d.lanes);
             // CSR-vector: sanitise placeholder columns outside the operand, keep the CSR arrays
             std::vector<int> colc(c.col);
             for (size_t k = 0; k < colc.size(); k++)

@@ -4,32 +4,114 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstddef>
 #include <vector>
 
 namespace layout {
 
+// Estimates of an FP64 sweep over a natural-order matrix, in cycles, for a group of S lanes per row (S = 1: one
+// thread per row).  A sweep is bound by the SM's FP64 units (19 cycles a warp instruction and SM, whatever its
+// active lanes: a warp's products are those of its longest row, then log2 S sums and two operations of the update)
+// or by the chain of the longest row (1,180 cycles per batch of eight entries, or of four strides: two L2 round
+// trips and the products).  Blocks of 256 threads do not divide evenly among 152 SMs: up to one and up to two blocks
+// an SM cost as much as one and two, more cost about one block an SM more than their number (the scheduler fills
+// some SMs further than others); for one thread per row, whose blocks are long, up to three cost 4.4.
+struct Rows {
+    long n = 0;
+    double avg = 0.0;
+    int longest = 0;
+    double products[6] = {}, warps[6] = {};  // per log2 S: products of the warps' longest rows, warps
+};
+
+inline Rows row_counts(int n, const int* ptr) {
+    Rows r;
+    r.n = n;
+    r.avg = n > 0 ? double(ptr[n] - ptr[0]) / n : 0.0;
+    int longest = 0;
+#pragma omp parallel for schedule(static) reduction(max : longest)
+    for (int i = 0; i < n; i++) longest = std::max(longest, ptr[i + 1] - ptr[i]);
+    r.longest = longest;
+    for (int lg = 0; lg < 6; lg++) {
+        if (lg == 1) continue;  // groups of two lanes are not used
+        const int S = 1 << lg, per = 32 / S;
+        const long warps = ((long)n + per - 1) / per;
+        double products = 0.0;
+#pragma omp parallel for schedule(static) reduction(+ : products)
+        for (long w = 0; w < warps; w++) {
+            int most = 0;
+            for (long i = w * per; i < std::min<long>(n, (w + 1) * per); i++) most = std::max(most, ptr[i + 1] - ptr[i]);
+            products += (most + S - 1) / S;
+        }
+        r.products[lg] = products;
+        r.warps[lg] = double(warps);
+    }
+    return r;
+}
+
+inline double sweep_cycles(const Rows& r, int lg) {
+    const int S = 1 << lg;
+    const double blocks = std::max(1.0, std::ceil(double(r.n) * S / 256.0)), L = blocks / 152.0;
+    const double full = L <= 1.0 ? 1.0 : L <= 2.0 ? 2.0 : lg == 0 && L < 3.0 ? 4.4 : L + 1.0;
+    const double pipe = full / L * (r.products[lg] + r.warps[lg] * (lg + 2)) * 19.0 / 152.0;
+    if (lg == 0) return 1500.0 + std::max(pipe, 1180.0 * ((r.longest + 7) / 8));
+    const double chain = 0.6 * (1180.0 * ((r.longest + 4 * S - 1) / (4 * S)) + 90.0 * lg);
+    // four lanes of long rows read half sectors of columns
+    return (1500.0 + std::max(pipe, chain)) * (lg == 2 && r.avg > 64.0 ? 1.1 : 1.0);
+}
+
+// Lanes per row of the FP64 passes over a natural-order matrix whose layout has `lanes` (the arrays are the same for
+// any number): those of the shortest estimate where it is under 0.85 of the layout's, for the estimates are good to
+// about 15 %.  Measured over 355 shapes (600 to 99,000 rows of 4 to 300 entries, even and skewed) and the 96 levels
+// of 17 hierarchies, GB300: on average 0.875 of the layout's lanes (the best choice: 0.86), 1.09 at worst (0.1 us);
+// without the margin and with mean instead of counted products up to 1.32 (32,000 rows of 158 entries: 4 lanes
+// 19.8 us, 8 lanes 15.0).  18,818 rows of 14 entries 4.8 (8 lanes) against 3.4 us (4), 13,011 of 94 8.8 (8)
+// against 7.2 (16), 3,196 of 4 to 119 5.9 (4) against 3.7 (16).
+inline int lanes64_for(const Rows& r, int lanes) {
+    int best = 2, own = 2;
+    for (int lg = 2; lg < 6; lg++) {
+        if (sweep_cycles(r, lg) < sweep_cycles(r, best)) best = lg;
+        if (1 << lg == lanes) own = lg;
+    }
+    return sweep_cycles(r, best) < 0.85 * sweep_cycles(r, own) ? 1 << best : lanes;
+}
+
+// Whether one thread per row suits a matrix of fewer than 100,000 rows (see lanes_for): not rows of more than
+// 192 entries or much longer ones among short ones (a slice of 32 rows is padded to its longest, a thread walks it
+// alone), nor, in natural order, where the estimate is longer than the lane groups'.  FP64 sweeps, one thread per
+// row against lane groups (the layout chosen): 33,282 rows of 14 entries (3.2 us) against 4.3, 50,748 of 53 (9.5)
+// against 10.0, 77,000 of 100 (16.8) against 23.5; 90,000 of 100 31.8 against (27.0), 45,000 of 200 29.2 against
+// (23.6); 90,000 rows of 8 with 300 in every 500th 29.8 against (15.8), in FP32 16.4 against (8.7).
+// lanes: the lane groups it would have otherwise.
+inline bool one_thread_suits(const Rows& r, bool grouped, int lanes) {
+    if (r.avg > 192.0 || r.longest > 3.0 * r.avg + 8.0) return false;
+    if (grouped) return true;
+    int lg = 2;
+    while (1 << lg < lanes64_for(r, lanes)) lg++;
+    return sweep_cycles(r, 0) <= 1.05 * sweep_cycles(r, lg);
+}
+
 // Layout choice, from sweeps of every level of elasticity (97 to 1,025 squared nodes) and Poisson hierarchies on
-// GB300 in every layout.  One thread per row (SELL-32; long rows software-pipelined) from 32,768 rows on: there
-// are enough of them, and each FP64 instruction, which costs an SM 19 cycles whatever its active lanes, does 32
-// rows' work (FP64 sweeps, one thread per row against 8 lanes per row: 34,814 rows of 8.5 entries 3.3 against
-// 6.9 us, 50,748 rows of 53 entries 9.9 against 14.8, 70,011 of 95 19.7 against 24.0, 34,046 of 113 14.9 against
-// 16.4; FP32 passes of such matrices read quads in either layout).  Below, a group of lanes per row, 8 lanes
-// from 8k rows (enough rows to fill the GPU, several loads in flight per lane), wider groups below.  A
-// colour-grouped matrix is swept colour by colour: its colours must have the rows to fill the GPU (groups: their
-// number), or, as before, 100,000 rows in all.  lean: the lane groups' CSR arrays, which hold no padding, up to
-// 100,000 rows (handles with a device-memory limit).  fused_rows: matrices of at most so many rows are read by fused
-// steps, which need lane groups (0: none are).  asked: the layout of lina_gpu_set_layout.
-// Returns the lanes per row, 0 for one thread per row.
-inline int lanes_for_shape(long n, double avg, long groups, bool lean, long fused_rows, int asked) {
+// GB300 in every layout.  One thread per row (SELL-32; long rows software-pipelined) from 100,000 rows on, and from
+// 32,768 (rows of fewer than 8 entries: from 24,577, where 31,000 of 5 take 2.1 us against 4.4) where it suits the
+// rows: there are enough of them, and each FP64 instruction does 32 rows' work (FP32 passes of such matrices read
+// quads in either layout).  Below, a group of lanes per row, 8 lanes from 8k rows (enough rows to fill the GPU,
+// several loads in flight per lane), wider groups below.  A colour-grouped matrix is swept colour by colour: its
+// colours must have the rows to fill the GPU (groups: their number), or it 100,000 rows in all.
+// n: the rows that the rule goes by (those of the largest system of a batch, or the matrix's).  lean: the lane
+// groups' CSR arrays, which hold no padding, up to 100,000 rows (handles with a device-memory limit).  fused_rows:
+// matrices of at most so many rows are read by fused steps, which need lane groups (0: none are).  asked: the
+// layout of lina_gpu_set_layout.  Returns the lanes per row, 0 for one thread per row.
+inline int lanes_for(long n, int rows, const int* ptr, long groups, bool lean, long fused_rows, int asked) {
     if (asked == 1) return 0;
     if (asked >= 3) return 4 << (asked - 3);
-    const bool many = n >= 100000 || (!lean && n > fused_rows &&
-                                      (groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768));
-    if (asked == 0 && many && avg <= 256.0) return 0;
-    if (avg < 8.0) return 4;
-    if (n >= 8000) return 8;
-    return avg >= 24.0 ? 16 : 8;
+    const double avg = rows > 0 ? double(ptr[rows] - ptr[0]) / rows : 0.0;
+    const int lanes = avg < 8.0 ? 4 : n >= 8000 ? 8 : avg >= 24.0 ? 16 : 8;
+    if (asked != 0 || avg > 256.0) return lanes;
+    if (n >= 100000) return 0;
+    const bool many = groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768 || (avg < 8.0 && n > 24576);
+    if (lean || n <= fused_rows || !many) return lanes;
+    return one_thread_suits(row_counts(rows, ptr), groups > 0, lanes) ? 0 : lanes;
 }
 
 // A fused step reads all four matrices of a level as CSR, by groups of so many lanes: the colour-grouped and the

@@ -422,7 +422,8 @@ int lina_gpu_free_host(void* p);
 int lina_gpu_device_count(void);
 int lina_gpu_set_device(int device);   /* select the GPU for hierarchies created afterwards */
 /* storage layout of matrices uploaded afterwards: 0 automatic (SELL-32 thread-per-row for levels of
-   100k rows or more, CSR with a lane group per row otherwise), 1 SELL-32 always, 2 CSR lane groups
+   100,000 rows or more, and from 32,768, short rows from 24,577, where rows are even and the estimate is no
+   slower; CSR with a lane group per row otherwise), 1 SELL-32 always, 2 CSR lane groups
    always (group size chosen from the mean row length), 3..6 CSR lane groups of 4, 8, 16 or 32 lanes (also in
    the colours of staged multicolour-SOR steps, which otherwise choose their FP64 lanes colour by colour) */
 int lina_gpu_set_layout(int layout);

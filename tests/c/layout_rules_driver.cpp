@@ -1,8 +1,12 @@
 // The layout rules (layout_rules.h) for tests without a GPU.
 #include "layout_rules.h"
 
-extern "C" int rule_lanes(long n, double avg, long groups, int lean, long fused_rows, int asked) {
-    return layout::lanes_for_shape(n, avg, groups, lean != 0, fused_rows, asked);
+extern "C" int rule_lanes(long n, int rows, const int* ptr, long groups, int lean, long fused_rows, int asked) {
+    return layout::lanes_for(n, rows, ptr, groups, lean != 0, fused_rows, asked);
+}
+
+extern "C" int rule_lanes64(int rows, const int* ptr, int lanes) {
+    return layout::lanes64_for(layout::row_counts(rows, ptr), lanes);
 }
 
 extern "C" int rule_fused(int acol, int a, int r, int p) { return layout::fused_layouts(acol, a, r, p) ? 1 : 0; }

@@ -23,19 +23,29 @@ def rules(tmp_path_factory):
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I" + os.path.join(ROOT, "fem_gb300", "csrc"),
                     os.path.join(ROOT, "tests", "c", "layout_rules_driver.cpp"), "-o", out], check=True)
     lib = C.CDLL(out)
-    lib.rule_lanes.argtypes = [C.c_long, C.c_double, C.c_long, C.c_int, C.c_long, C.c_int]
+    lib.rule_lanes.argtypes = [C.c_long, C.c_int, C.c_void_p, C.c_long, C.c_int, C.c_long, C.c_int]
+    lib.rule_lanes64.argtypes = [C.c_int, C.c_void_p, C.c_int]
     return lib
+
+
+def pointers(n, lengths):
+    """Row pointers of n rows whose lengths repeat."""
+    return np.concatenate(([0], np.cumsum(np.resize(np.asarray(lengths, np.int64), n)))).astype(np.int32)
+
+
+def lanes(rules, n, lengths, groups=0, lean=0, fused=24576, asked=0):
+    ptr = pointers(n, lengths)
+    return rules.rule_lanes(n, n, ptr.ctypes.data, groups, lean, fused, asked)
 
 
 def test_fused_steps_need_lane_groups_everywhere(rules):
     """A three-coloured level of 33,000 rows of three entries: its colours keep lane groups where its natural-order
     matrix and its prolongation take one thread per row, so no fused step may read them in lane groups."""
-    acol, a, p, r = (rules.rule_lanes(*s, 0, 24576, 0) for s in ((33000, 3.0, 3), (33000, 3.0, 0), (33000, 1.5, 0), (11000, 3.0, 0)))
+    acol, a, p, r = lanes(rules, 33000, [3], 3), lanes(rules, 33000, [3]), lanes(rules, 33000, [1, 2]), lanes(rules, 11000, [3])
     assert acol > 0 and a == 0 and p == 0 and r > 0
     assert not rules.rule_fused(acol, a, r, p)
     for k in range(16):
-        lanes = [8 * (k >> i & 1) for i in range(4)]
-        assert bool(rules.rule_fused(*lanes)) == (k == 15)
+        assert bool(rules.rule_fused(*[8 * (k >> i & 1) for i in range(4)])) == (k == 15)
 
 
 def test_levels_within_the_row_limit_keep_lane_groups(rules):
@@ -43,20 +53,51 @@ def test_levels_within_the_row_limit_keep_lane_groups(rules):
     for limit in (24576, 32768, 33000, 49152, 99999):
         for n in (1000, 24576, 32767, 32768, 33000, 49152, 99999):
             if n <= limit:
-                lanes = [rules.rule_lanes(n, avg, g, 0, limit, 0) for avg, g in ((3.0, 3), (14.0, 2), (3.0, 0), (60.0, 0))]
-                assert min(lanes) > 0, (n, limit)
-        assert rules.rule_lanes(limit + 1, 14.0, 0, 0, limit, 0) == (0 if limit + 1 >= 32768 else 8)
+                assert min(lanes(rules, n, [k], g, fused=limit) for k, g in ((3, 3), (14, 2), (3, 0), (60, 0))) > 0
+        assert lanes(rules, limit + 1, [3], fused=limit) == 0
+        assert lanes(rules, limit + 1, [14], fused=limit) == (0 if limit + 1 >= 32768 else 8)
+
+
+def test_one_thread_per_row_only_where_it_is_no_slower(rules):
+    """32,768 to 100,000 rows: even rows that fill the SMs take one thread per row; long rows among short ones, and row
+    counts whose blocks divide badly among the SMs, keep the lane groups that measured faster."""
+    for n, k in ((32768, 14), (33282, 14), (50748, 53), (66188, 53), (66049, 7), (75975, 95), (77000, 100), (99000, 5),
+                 (31000, 5), (24577, 7)):
+        assert lanes(rules, n, [k]) == 0, (n, k)
+    for n, rows in ((24576, [5]), (31000, [8]), (36000, [250]), (45000, [200]), (80000, [100]), (90000, [60]), (90000, [200]),
+                    (36000, [8] * 499 + [300]), (90000, [8] * 499 + [300]), (65000, [20] * 49 + [200]),
+                    (90000, [4] * 4999 + [1500]), (45000, [60] * 49 + [250])):
+        assert lanes(rules, n, rows) > 0, (n, rows[0])
+    assert lanes(rules, 66000, [7], 4) == 0 and lanes(rules, 66000, [4] * 99 + [60], 4) > 0
+    # at and above 100,000 rows, and in every asked-for layout, as before
+    assert lanes(rules, 100000, [8] * 499 + [300]) == 0 and lanes(rules, 100000, [257]) == 8
+    assert lanes(rules, 99999, [14], lean=1) == 8
+    assert [lanes(rules, 50000, [14], asked=k) for k in range(1, 7)] == [0, 8, 4, 8, 16, 32]
+
+
+def test_fp64_lanes_change_only_for_a_clear_gain(rules):
+    """Other lanes than the layout's where they measured well under its time, the layout's where they measured over it."""
+    def lanes64(n, rows, own):
+        ptr = pointers(n, rows)
+        return rules.rule_lanes64(n, ptr.ctypes.data, own)
+    assert lanes64(18818, [14], 8) == 4 and lanes64(9214, [22], 8) == 4
+    for n, k in ((24000, 100), (24000, 160), (32000, 130), (32000, 160), (32000, 200), (65000, 160), (9000, 80)):
+        assert lanes64(n, [k], 8) == 8, (n, k)
+    assert lanes64(90000, [4] * 9 + [16], 4) == 4 and lanes64(5000, [4] * 9 + [16], 4) == 4
+    assert lanes64(2000, [4] * 999 + [700], 4) == 32
+    for n in (0, 1, 31):
+        assert lanes64(n, [1], 4) in (4, 8, 16, 32)
 
 
 def test_layouts_asked_for_win(rules):
     """lina_gpu_set_layout(3..6) fixes the lanes of the staged colours as well, 1 keeps a batch's levels out of lane
     groups; 0 and 2 leave both to the rules."""
     few, many = np.array([300, 280, 4], np.int32), np.full(4000, 7, np.int32)
-    lanes = lambda v, n, asked: rules.rule_stage_lanes(v.ctypes.data_as(C.c_void_p), len(v), n, asked)  # noqa: E731
+    stage = lambda v, n, asked: rules.rule_stage_lanes(v.ctypes.data_as(C.c_void_p), len(v), n, asked)  # noqa: E731
     for asked in (3, 4, 5, 6):
-        assert lanes(few, 4 << (asked - 3), asked) == lanes(many, 4 << (asked - 3), asked) == 4 << (asked - 3)
+        assert stage(few, 4 << (asked - 3), asked) == stage(many, 4 << (asked - 3), asked) == 4 << (asked - 3)
     for asked in (0, 2):
-        assert lanes(few, 8, asked) == 32 and lanes(many, 8, asked) == 1
+        assert stage(few, 8, asked) == 32 and stage(many, 8, asked) == 1
     assert [rules.rule_groups_allowed(k) for k in range(7)] == [1, 0, 1, 1, 1, 1, 1]
 
 
