@@ -88,7 +88,6 @@ void set_err(const char* fmt, ...) {
 
 constexpr int kThreads = 256;
 constexpr int kMaxBlocks = 16384;     // partials per reduction value
-constexpr int kFewRows = 152 * 4 * kThreads;  // one wave of sell_kernel's R_FEW variant
 constexpr int kGridCap = 152 * 12;    // grid-stride cap: 152 SMs x 12 blocks of 256
 constexpr int kReduceGrid = 152 * 4;  // streaming reductions: half a wave, four strides per loop trip
 
@@ -274,9 +273,12 @@ __device__ __forceinline__ int sell_col(unsigned short d, int2 base) {
 
 // rowseg / act (segmented batches, else null): the system of every row and whether it is still iterating;
 // the rows of systems that have stopped are skipped (their values are not used any more)
-enum { R_SHORT = 0, R_FEW = 1, R_LONG = 2 };
+using layout::SELL_FEW;
+using layout::SELL_LONG;
+using layout::SELL_LONG_EARLY;
+using layout::SELL_SHORT;
 template <typename TV, typename TX, int MODE, int ROWS, typename TI>
-__global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel(int npos, int nrows, const int* __restrict__ rowmap,
+__global__ void __launch_bounds__(kThreads, ROWS == SELL_FEW || ROWS == SELL_LONG_EARLY ? 4 : 0) sell_kernel(int npos, int nrows, const int* __restrict__ rowmap,
                                                         const int* __restrict__ sptr, const int2* __restrict__ sbase,
                                                         const TI* __restrict__ col, const TV* __restrict__ val,
                                                         const TX* x, TX* y, const TX* __restrict__ b,
@@ -287,9 +289,9 @@ __global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel
     // grid-stride over slice positions (npos is a multiple of 32, so warps stay whole); positions
     // past the last row (natural order) or marked -1 (colour order) are padding
     int t = blockIdx.x * blockDim.x + threadIdx.x;
-    // The matrix does not change while kernels run, so a thread's first row and (R_FEW, R_LONG) its first batch of
-    // eight entries are loaded before it waits for the previous kernel.
-    constexpr bool EARLY = ROWS != R_SHORT;
+    // The matrix does not change while kernels run, so a thread's first row and (SELL_FEW, SELL_LONG_EARLY) its first
+    // batch of eight entries are loaded before it waits for the previous kernel.
+    constexpr bool EARLY = ROWS == SELL_FEW || ROWS == SELL_LONG_EARLY;
     TI c[8];
     TV v[8];
     bool waited = !EARLY;
@@ -329,7 +331,7 @@ __global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel
         if constexpr (EARLY) {
             if (len >= 8)
                 fetch(0);
-            else if constexpr (ROWS == R_FEW)
+            else if constexpr (ROWS == SELL_FEW)
                 fetch_rest(0);
             if (!waited) {
                 pdl_wait();
@@ -342,15 +344,9 @@ __global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel
         // thread keeps several loads in flight.  x is read through the read-only path (no thread reads an entry
         // of y written by another thread of the same launch, also in the in-place SOR mode, where rows of one
         // colour do not couple).
-        //  R_LONG (dense coarse operators): software-pipelined, the indices and values of the next batch are
-        //   loaded before the products of the current one.
-        //  R_SHORT: 32 registers, so that 64 warps an SM hide the latency.
-        //  R_FEW (short rows, at most a wave of blocks): latency is what counts, so the rest of a row after its
-        //   batches is loaded together, predicated, in 64 registers.  Measured on GB300: a segmented batch whose
-        //   colour launches are such 94 ms with R_SHORT, 80 ms with R_FEW; a sweep of 2.1M rows of 14 entries
-        //   in FP64 82 us with R_SHORT, 88 us with R_FEW.
+        // layout::sell_variant says which variant suits which rows.
         int k = 0;
-        if constexpr (ROWS == R_FEW) {
+        if constexpr (ROWS == SELL_FEW) {
             if (len >= 8) {
                 for (k = 8;; k += 8) {
                     TX xv[8];
@@ -369,13 +365,25 @@ __global__ void __launch_bounds__(kThreads, ROWS == R_SHORT ? 0 : 4) sell_kernel
 #pragma unroll
                 for (int u = 0; u < 7; u++)
                     if (k + u < len) xv[u] = __ldg(x + sell_col(c[u], cb));
+                if constexpr (sizeof(TX) == 8) {
+                    // branches (a warp's rows are of one length), not predicates (see csrv_kernel): 105,000 rows of
+                    // 9 entries 6.1 -> 4.8 us, of 6 with 17 in every tenth 8.3 -> 7.0
 #pragma unroll
-                for (int u = 0; u < 7; u++)
-                    if (k + u < len) sum += TX(v[u]) * xv[u];
+                    for (int u = 0; u < 7; u++) {
+                        if (k + u >= len) break;
+                        asm volatile("" ::: "memory");
+                        sum += TX(v[u]) * xv[u];
+                    }
+                } else {
+#pragma unroll
+                    for (int u = 0; u < 7; u++)
+                        if (k + u < len) sum += TX(v[u]) * xv[u];
+                }
                 k = len;
             }
-        } else if constexpr (ROWS == R_LONG) {
+        } else if constexpr (ROWS == SELL_LONG || ROWS == SELL_LONG_EARLY) {
             if (len >= 8) {
+                if constexpr (!EARLY) fetch(0);
                 for (k = 8;; k += 8) {
                     TX xv[8];
 #pragma unroll
@@ -2614,12 +2622,14 @@ struct lina_gpu_amg {
             launch(sell_kernel<TV, TX, MODE, R, int>, gd, bd, 0, stream, npos, nrows, rm, sp, sb,                  \
                    (const int*)m.col, val, x, y, b, dinv, w, z, partials, ticket, sc, rseg, m.act);                \
     } while (0)
-        if (m.long_rows)
-            LINA_SELL(R_LONG);
-        else if (npos <= kFewRows)
-            LINA_SELL(R_FEW);
-        else
-            LINA_SELL(R_SHORT);
+        switch (layout::sell_variant(sizeof(TX) == 8, m.long_rows, npos)) {
+            case SELL_SHORT: LINA_SELL(SELL_SHORT); break;
+            case SELL_FEW: LINA_SELL(SELL_FEW); break;
+            case SELL_LONG_EARLY: LINA_SELL(SELL_LONG_EARLY); break;
+            case SELL_LONG:
+                if constexpr (sizeof(TX) == 4) LINA_SELL(SELL_LONG);
+                break;
+        }
 #undef LINA_SELL
         if (MODE == M_DOT) launch(dot_finish_kernel, dim3(1), dim3(dot_finish_threads(grid)), 0, stream, grid, (const double*)partials, sc);
     }

@@ -81,7 +81,7 @@ inline int lanes64_for(const Rows& r, int lanes) {
 // alone), nor, in natural order, where the estimate is longer than the lane groups'.  FP64 sweeps, one thread per
 // row against lane groups (the layout chosen): 33,282 rows of 14 entries (3.2 us) against 4.3, 50,748 of 53 (9.5)
 // against 10.0, 77,000 of 100 (16.8) against 23.5; 90,000 of 100 31.8 against (27.0), 45,000 of 200 29.2 against
-// (23.6); 90,000 rows of 8 with 300 in every 500th 29.8 against (15.8), in FP32 16.4 against (8.7).
+// (23.6); 90,000 rows of 8 with 300 in every 500th 29.8 against (15.8), in FP32 without quads 16.4 against (8.7).
 // lanes: the lane groups it would have otherwise.
 inline bool one_thread_suits(const Rows& r, bool grouped, int lanes) {
     if (r.avg > 192.0 || r.longest > 3.0 * r.avg + 8.0) return false;
@@ -112,6 +112,22 @@ inline int lanes_for(long n, int rows, const int* ptr, long groups, bool lean, l
     const bool many = groups > 0 ? avg < 24.0 && n >= 16384 * groups : n >= 32768 || (avg < 8.0 && n > 24576);
     if (lean || n <= fused_rows || !many) return lanes;
     return one_thread_suits(row_counts(rows, ptr), groups > 0, lanes) ? 0 : lanes;
+}
+
+// Variants of the one-thread-per-row kernel (sell_kernel) for a launch of npos rows.  SHORT rows in 32 registers, so
+// that 64 warps an SM hide the latency; FEW of them with the rest of a row loaded together and the first entries
+// before the wait for the previous kernel; LONG rows (mean of 24 and more) software-pipelined, with those first loads
+// (EARLY) or without.  FEW pays up to a wave of its blocks, four an SM: repeated FP32 sweeps of 33,000 rows of 14
+// entries 3.4 us SHORT, 2.0 FEW, of 155,000 3.9 and 2.9; a segmented batch 94 and 80 ms; a solve of 101,250 rows in
+// FP64 5.83 and 5.30 ms, though repeated FP64 sweeps of such rows alone take 5.4 SHORT and 6.2 FEW.  (2.1M rows of 14
+// in FP64: 82 us SHORT, 88 FEW.)  EARLY in FP32 takes registers: it wins up to a block an SM (33,000 rows of 30 4.3
+// against 3.8 us, of 100 6.8 against 6.5; 50,000 of 100 7.4 against 8.5, 105,000 of 60 8.0 against 9.7), in FP64 it
+// does not lose (33,000 of 30 5.4 against 4.9, 250,000 of 60 38 against 35).
+enum SellVariant { SELL_SHORT = 0, SELL_FEW = 1, SELL_LONG = 2, SELL_LONG_EARLY = 3 };
+constexpr long kBlockRows = 152L * 256;  // rows of one block on each SM
+inline SellVariant sell_variant(bool f64, bool long_rows, long npos) {
+    if (long_rows) return f64 || npos <= kBlockRows ? SELL_LONG_EARLY : SELL_LONG;
+    return npos <= 4 * kBlockRows ? SELL_FEW : SELL_SHORT;
 }
 
 // A fused step reads all four matrices of a level as CSR, by groups of so many lanes: the colour-grouped and the

@@ -16,3 +16,7 @@ extern "C" int rule_stage_lanes(const int* len, int count, int lanes, int asked)
 }
 
 extern "C" int rule_groups_allowed(int asked) { return layout::groups_allowed(asked) ? 1 : 0; }
+
+extern "C" int rule_sell_variant(int f64, int long_rows, long npos) {
+    return (int)layout::sell_variant(f64 != 0, long_rows != 0, npos);
+}

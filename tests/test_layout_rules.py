@@ -13,6 +13,7 @@ import scipy.sparse as sp
 
 from fem_gb300 import lina, problems
 from tests.conftest import ROOT, gpu_available
+from tests.test_layouts import matrix
 
 gpu = pytest.mark.skipif(not gpu_available(), reason="no CUDA device")
 
@@ -25,6 +26,7 @@ def rules(tmp_path_factory):
     lib = C.CDLL(out)
     lib.rule_lanes.argtypes = [C.c_long, C.c_int, C.c_void_p, C.c_long, C.c_int, C.c_long, C.c_int]
     lib.rule_lanes64.argtypes = [C.c_int, C.c_void_p, C.c_int]
+    lib.rule_sell_variant.argtypes = [C.c_int, C.c_int, C.c_long]
     return lib
 
 
@@ -101,12 +103,46 @@ def test_layouts_asked_for_win(rules):
     assert [rules.rule_groups_allowed(k) for k in range(7)] == [1, 0, 1, 1, 1, 1, 1]
 
 
+def test_sell_variants_by_blocks_per_sm(rules):
+    """Short, few, long, long with early loads (0 to 3), either side of one and four blocks of 256 rows an SM."""
+    v = rules.rule_sell_variant
+    assert [v(f64, 0, n) for f64 in (0, 1) for n in (32, 155648, 155680)] == [1, 1, 0, 1, 1, 0]
+    assert [v(1, 1, n) for n in (32, 38944, 1 << 20)] == [3, 3, 3]
+    assert [v(0, 1, n) for n in (32, 38912, 38944, 1 << 20)] == [3, 3, 2, 2]
+
+
 def ring(n):
     """Periodic second differences with a shift."""
     e = np.ones(n)
     A = sp.diags([2.1 * e, -e[:-1], -e[:-1], -1.0, -1.0], [0, 1, -1, n - 1, 1 - n], format="csr")
     A.sort_indices()
     return A
+
+
+@gpu
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", [lina.PREC_FP64, lina.PREC_MIXED])
+@pytest.mark.parametrize("n,lengths", [(155648, range(0, 18)), (155649, range(0, 18)), (38912, [23, 26, 40]),
+                                       (38913, [23, 26, 40])])
+def test_sell_variants_at_their_edges(n, lengths, prec):
+    """Products and sweeps of the one-entry SELL layout either side of the variants' row counts.  Bar: k products summed
+    in any order in a format of unit roundoff u are off by at most (k + 2) u |A| |x|, the update by a few u more."""
+    A = matrix(n, list(lengths), n)
+    lina.set_layout(1)
+    lina.set_sell_quads(0)
+    try:
+        M = lina.Matrix(n, A.indptr, A.indices, A.data)
+    finally:
+        lina.set_layout(0)
+        lina.set_sell_quads(1)
+    u, dt = (2.0 ** -24, np.float32) if prec == lina.PREC_MIXED else (2.0 ** -53, np.float64)
+    rng = np.random.default_rng(7)
+    x, b = rng.uniform(-1, 1, n).astype(dt), rng.uniform(-1, 1, n).astype(dt)
+    x64, b64 = x.astype(np.float64), b.astype(np.float64)
+    S, k, d = abs(A) @ abs(x64), np.diff(A.indptr), 1.0 / A.diagonal()
+    assert (np.abs(M.spmv(x, prec) - A @ x64) <= (k + 4) * u * S).all()
+    ref = x64 + 0.6 * d * (b64 - A @ x64)
+    assert (np.abs(M.jacobi(b, x, 0.6, 1, prec) - ref) <= 0.6 * d * (k + 8) * u * (S + abs(b64)) + 4 * u * abs(x64)).all()
 
 
 @gpu
