@@ -343,8 +343,8 @@ __global__ void strip_entries_kernel(long ne, const int* __restrict__ enc, const
                                      strip::Entry<double>* __restrict__ e64, strip::Entry<float>* __restrict__ e32) {
     for (long q = (long)blockIdx.x * blockDim.x + threadIdx.x; q < ne; q += (long)gridDim.x * blockDim.x) {
         const int p = perm[q], at = enc[q];  // p -1: padding
-        e64[q] = strip::Entry<double>{8u * at, 0u, p >= 0 ? plain_nan(v64[p]) : 0.0};
-        e32[q] = strip::Entry<float>{4u * at, p >= 0 ? plain_nan(v32[p]) : 0.0f};
+        if (e64) e64[q] = strip::Entry<double>{8u * at, 0u, p >= 0 ? plain_nan(v64[p]) : 0.0};
+        if (e32) e32[q] = strip::Entry<float>{4u * at, p >= 0 ? plain_nan(v32[p]) : 0.0f};
     }
 }
 
@@ -353,8 +353,8 @@ __global__ void strip_points_kernel(int n, const int* __restrict__ row, const do
                                     strip::Point<float>* __restrict__ p32) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int i = row[t];
-        p64[t] = strip::Point<double>{i, 0, i >= 0 && d64 ? plain_nan(d64[i]) : 1.0};
-        p32[t] = strip::Point<float>{i, i >= 0 && d32 ? plain_nan(d32[i]) : 1.0f};
+        if (p64) p64[t] = strip::Point<double>{i, 0, i >= 0 && d64 ? plain_nan(d64[i]) : 1.0};
+        if (p32) p32[t] = strip::Point<float>{i, i >= 0 && d32 ? plain_nan(d32[i]) : 1.0f};
     }
 }
 
@@ -582,8 +582,9 @@ struct Factor {
         double *val64 = nullptr, *dinv64 = nullptr;
         float *val32 = nullptr, *dinv32 = nullptr;
     } win;
-    // the solve pipelined over strips (strips = 0: one of the other two)
+    // the solve pipelined over strips (strips = 0: one of the other two), in the precisions it pays in
     struct Strips {
+        bool use32 = false, use64 = false;
         int strips = 0, ring = 0, width = 0, max_width = 0;
         int npos = 0;
         long ne = 0;
@@ -841,26 +842,36 @@ bool upload_window(lina_gpu_ilu* h, Factor& f, const WinPlan& pl, bool has_dinv)
     return true;
 }
 
-// How a factor is solved: pipelined over strips where its plan exists (strip::make_plan says which
-// matrices suit it), else by one block walking the levels where a level fits its shared memory, else by
-// the row pool.  ILU(0) of the AT2 damage matrix on GB300, one application (two solves):
+// How a factor is solved, precision by precision: pipelined over strips where its plan exists (strip::make_plan
+// says which matrices suit it) and is no slower than the one block (strip::pays), else by one block walking the
+// levels where a level fits its shared memory, else over the strips if there is a plan, else by the row pool.  ILU(0) of the AT2 damage matrix on GB300, one application (two solves):
 //   1025 x 1025 nodes, FP32: one block 2.87 ms, strips 0.52 ms
 //    389 x 389 nodes, FP64: one block 1.20 ms, strips 0.45 ms
 struct SolvePlan {
     strip::Plan strips;
     WinPlan window;
+    bool use32 = false, use64 = false;  // the strips are used in that precision
 };
 
 void plan_solve(SolvePlan& pl, int n, const std::vector<int>& order, const std::vector<int>& lev,
                 const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end, const int* col,
                 bool has_dinv, bool lower) {
-    if (!strip::make_plan(pl.strips, n, order, lev, (int)lp.size() - 1, beg, end, col, lower))
-        plan_window(pl.window, n, order, lev, lp, beg, end, col, has_dinv);
+    const bool plan = strip::make_plan(pl.strips, n, order, lev, (int)lp.size() - 1, beg, end, col, lower);
+    pl.use32 = plan && strip::pays(pl.strips, false);
+    pl.use64 = plan && strip::pays(pl.strips, true);
+    if (pl.use32 && pl.use64) return;
+    plan_window(pl.window, n, order, lev, lp, beg, end, col, has_dinv);
+    if (!plan) return;
+    pl.use32 = pl.use32 || !pl.window.w.s32;
+    pl.use64 = pl.use64 || !pl.window.w.s64;
+    if (!pl.use32 && !pl.use64) pl.strips = strip::Plan();
 }
 
 bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl, bool has_dinv) {
     const strip::Plan& p = pl.strips;
-    if (!p.strips) return upload_window(h, f, pl.window, has_dinv);
+    if (!p.strips || !pl.use32 || !pl.use64)
+        if (!upload_window(h, f, pl.window, has_dinv)) return false;
+    if (!p.strips) return true;
     Factor::Strips& w = f.strip;
     Mem& m = h->mem;
     w = Factor::Strips();
@@ -876,15 +887,23 @@ bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl, bool has_dinv
     w.row = m.up(p.row);
     w.enc = m.up(p.enc);
     w.perm = m.up(p.perm);
-    w.entry64 = m.get<strip::Entry<double>>(w.ne);
-    w.entry32 = m.get<strip::Entry<float>>(w.ne);
-    w.point64 = m.get<strip::Point<double>>(w.npos);
-    w.point32 = m.get<strip::Point<float>>(w.npos);
-    bool ok = w.first && w.ext_first && w.ext && w.table && w.row && w.enc && w.perm && w.entry64 &&
-              w.entry32 && w.point64 && w.point32;
+    bool ok = w.first && w.ext_first && w.ext && w.table && w.row && w.enc && w.perm;
+    if (pl.use64) {
+        w.entry64 = m.get<strip::Entry<double>>(w.ne);
+        w.point64 = m.get<strip::Point<double>>(w.npos);
+        ok = ok && w.entry64 && w.point64;
+    }
+    if (pl.use32) {
+        w.entry32 = m.get<strip::Entry<float>>(w.ne);
+        w.point32 = m.get<strip::Point<float>>(w.npos);
+        ok = ok && w.entry32 && w.point32;
+    }
     ok = ok && ensure_positions(h, w.npos);
-    if (ok) w.strips = p.strips;
-    return ok;
+    if (!ok) return false;
+    w.strips = p.strips;
+    w.use32 = pl.use32;
+    w.use64 = pl.use64;
+    return true;
 }
 
 bool build_solve(lina_gpu_ilu* h, Factor& f, int n, const std::vector<int>& order, const std::vector<int>& lev,
@@ -902,7 +921,6 @@ void pack_solve(Factor& f, int n) {
         const int ge = (int)std::min<long>(4096, (w.ne + kT - 1) / kT), gp = std::min(4096, (w.npos + kT - 1) / kT);
         strip_entries_kernel<<<ge, kT, 0, st()>>>(w.ne, w.enc, w.perm, f.val64, f.val32, w.entry64, w.entry32);
         strip_points_kernel<<<gp, kT, 0, st()>>>(w.npos, w.row, f.dinv64, f.dinv32, w.point64, w.point32);
-        return;
     }
     Factor::Win& w = f.win;
     if (!w.s32 && !w.s64) return;
@@ -1146,7 +1164,7 @@ void solve_strips(lina_gpu_ilu* h, const Factor& f, const TX* dinv, const TB* b,
 
 template <typename TV, typename TX>
 void solve(lina_gpu_ilu* h, const Factor& f, const TV* val, const TX* dinv, const TX* b, TX* x) {
-    if (f.strip.strips) {
+    if (sizeof(TX) == 8 ? f.strip.use64 : f.strip.use32) {
         solve_strips<TX, TX>(h, f, dinv, b, x);
         return;
     }
@@ -1422,7 +1440,7 @@ int lina_gpu_ilu_apply(lina_gpu_ilu* h, int precision, const double* r_dev, doub
     const int n = h->n;
     const int g = (int)std::min<long>(2048, (n + kT - 1) / kT);
     if (precision == LINA_PREC_MIXED) {
-        if (h->L.strip.strips) {
+        if (h->L.strip.use32) {
             solve_strips<float, double>(h, h->L, h->L.dinv32, r_dev, h->t32);
         } else {
             cvt_kernel<double, float><<<g, kT, 0, st()>>>(n, r_dev, h->r32);

@@ -25,7 +25,7 @@ constexpr int kMaxStrips = 148;            // one block per SM, a few left free
 constexpr int kRowsPerStrip = 30;          // rows of the widest level per strip: a step holds 32
 constexpr int kMaxEntries = 16;            // entries of a row (stage size)
 constexpr int kSmemMax = 200 * 1024;
-constexpr int kLag = 25;                   // steps an exchange between strips takes (about 2 us)
+constexpr int kLag = 25;                   // steps an exchange between strips takes, about (2 us, in FP32)
 
 // The plan of one factor: positions are chunk * 256 + step * 32 + lane.
 struct Plan {
@@ -34,6 +34,8 @@ struct Plan {
     int ring = 0;        // steps kept (a power of two)
     int width = 0;       // entries per row of every chunk where that is at most 4, else 0 (table)
     int max_width = 0;
+    double ns32 = 0.0, ns64 = 0.0;     // estimated time of a solve in FP32, in FP64
+    double win32 = 0.0, win64 = 0.0;   // and of the one-block solve of the same levels
     std::vector<int> first;            // first chunk of each strip (strips + 1)
     std::vector<int> ext_first;        // first fetched entry of each strip (strips + 1)
     std::vector<int> ext;              // row of each fetched entry
@@ -44,6 +46,27 @@ struct Plan {
     size_t positions() const { return (size_t)chunks * kPos; }
 };
 
+// Times on GB300 in ns.  A step of w entries a row, held in registers (fixed: every row has w <= 4 of them) or read where
+// they are used (in groups of four and singly): from chains of 20,000 and 400 levels of 16 rows.  A level of the
+// one-block solve whose rows have up to e entries: the same chains (levels of more rows take longer; so an estimate
+// below it is a gain; only rows of mostly 8 or 16 entries are counted longer, whose entries lie a multiple of the banks
+// apart: 128 rows of 8 take 0.19 us a level more, of 16 0.8).  An exchange between strips takes 2.4 us.
+constexpr double kLagNs = 2400.0;
+inline double step_ns(int w, bool fixed, bool f64) {
+    if (fixed) return f64 ? 76.0 + 43.0 * w : 62.0 + 4.5 * w;
+    return f64 ? 110.0 + 197.0 * (w / 4) + 58.0 * (w % 4) : 110.0 + 40.0 * (w / 4) + 55.0 * (w % 4);
+}
+inline double level_ns(int e, bool f64) {
+    constexpr double t32[kMaxEntries + 1] = {540, 550, 580, 580, 655, 680, 684, 715, 752,
+                                             752, 753, 754, 755, 780, 820, 850, 879};
+    constexpr double t64[kMaxEntries + 1] = {600,  606,  685,  685,  861,  879,  881,  1040, 1216,
+                                             1217, 1218, 1219, 1220, 1220, 1220, 1220, 1930};
+    return f64 ? t64[e] : t32[e];
+}
+inline double conflict_ns(int e, int rows, long entries) {
+    return (e == 8 || e == 16) && entries >= 0.9 * e * rows ? (e == 8 ? 0.12 : 0.33) * entries : 0.0;
+}
+
 // Rows listed level by level (order, with lev[i] the level of row i, nlev levels), row i's entries
 // [beg_i, end_i) of col.  lower: a row needs smaller indices.  Returns false (no plan) where
 //  - the widest level has more than 4,440 rows: the levels are wide enough for the other solves;
@@ -51,8 +74,8 @@ struct Plan {
 //  - more than 8 entries per step come from other strips, which the helper warps could not fetch in
 //    the time of a step (64 lanes, an L2 round trip each);
 //  - a chunk has more than 256 fetched entries (it and the next one share the slots);
-//  - the pipeline, followed step by step, takes more than 4 steps per level: a step is about 0.05 us in
-//    FP32 and 0.15 us in FP64, a level of the one-block solve 0.3 us and more.
+//  - the pipeline, followed step by step with an exchange of kLag steps, takes more than 4 steps per level.
+// Whether it is faster than the one-block solve, where there is one, its estimates say (pays).
 inline bool make_plan(Plan& P, int n, const std::vector<int>& order, const std::vector<int>& lev, int nlev,
                       const std::vector<int>& beg, const std::vector<int>& end, const int* col, bool lower) {
     P = Plan();
@@ -164,27 +187,54 @@ inline bool make_plan(Plan& P, int n, const std::vector<int>& order, const std::
     P.ext.resize(P.ext_first[K]);
     for (int s = 0; s < K; s++) std::copy(ext[s].begin(), ext[s].end(), P.ext.begin() + P.ext_first[s]);
     if ((long)P.ext.size() > 8 * steps) return false;
-    // the pipeline in units of a step: a step starts when the one before it and its chunk's fetched entries are
-    // there
-    std::vector<std::vector<long>> done(K);
-    long last = 0;
+    // the pipeline in units of a step, and in ns: a step starts when the one before it and its chunk's fetched entries
+    // are there
+    struct Time {
+        double v[3];
+    };
+    std::vector<std::vector<Time>> done(K);
+    Time last = {};
+    const double lag[3] = {kLag, kLagNs, kLagNs};
     for (int s = 0; s < K; s++) {
-        done[s].assign(nsteps[s], 0);
+        done[s].assign(nsteps[s], Time{});
         size_t e = 0;
-        long now = 0;
+        Time now = {};
         for (int step = 0; step < nsteps[s]; step++) {
             for (; e < ext[s].size() && ext_step[s][e] / kSteps == step / kSteps; e++) {
                 const int j = ext[s][e];
-                now = std::max(now, done[strip_of(j)][stepof[j] / 32] + kLag);
+                for (int k = 0; k < 3; k++) now.v[k] = std::max(now.v[k], done[strip_of(j)][stepof[j] / 32].v[k] + lag[k]);
             }
-            done[s][step] = ++now;
+            const int w = P.table[4 * (size_t)(P.first[s] + step / kSteps) + 1];
+            now.v[0] += 1.0;
+            now.v[1] += step_ns(w, P.width > 0, false);
+            now.v[2] += step_ns(w, P.width > 0, true);
+            done[s][step] = now;
         }
-        last = std::max(last, now);
+        for (int k = 0; k < 3; k++) last.v[k] = std::max(last.v[k], now.v[k]);
     }
-    if (last > 4L * nlev + 4L * kLag) return false;
+    if (last.v[0] > 4.0 * nlev + 4.0 * kLag) return false;
+    P.ns32 = last.v[1];
+    P.ns64 = last.v[2];
+    std::vector<int> most(nlev, 0);
+    std::vector<long> entries(nlev, 0);
+    for (int i = 0; i < n; i++) {
+        most[lev[i]] = std::max(most[lev[i]], end[i] - beg[i]);
+        entries[lev[i]] += end[i] - beg[i];
+    }
+    for (int l = 0; l < nlev; l++) {
+        P.win32 += level_ns(most[l], false) + conflict_ns(most[l], width[l], entries[l]);
+        P.win64 += level_ns(most[l], true) + conflict_ns(most[l], width[l], entries[l]);
+    }
     P.strips = K;
     return true;
 }
+
+// Whether the strips are used where the one-block solve is there too.  Most mesh matrices gain 2 to 5 times in either
+// precision (5-, 7- and 9-point grids, Delaunay meshes, interleaved components).  Few do not: levels that cross few
+// strips, so that a strip walks several steps of each (four strips of 100 lines of 120 points, coupled to the
+// line before by e points: FP64 569 us one block, 656 strips for e = 3, 722 and 1,163 for 5, 1,003 and 2,174 for
+// 12; FP32 478 and 228, 557 and 677, 685 and 776).
+inline bool pays(const Plan& P, bool f64) { return f64 ? P.ns64 <= P.win64 : P.ns32 <= P.win32; }
 
 // ---------------------------------------------------------------- the ILU(0) factorisation on the strips
 // A row of the factorisation needs the upper entries U_kj of the rows k its lower entries name: the
