@@ -3929,6 +3929,7 @@ int read_scalars(lina_gpu_amg* h) {
 namespace lina {
 namespace dev {
 void set_error(const char* msg) { g_err = msg ? msg : ""; }
+long memory_limit() { return g_mem_limit; }
 }  // namespace dev
 }  // namespace lina
 

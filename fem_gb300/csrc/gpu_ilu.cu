@@ -599,12 +599,24 @@ struct Factor {
 
 struct Mem {
     std::vector<void*> p;
+    size_t bytes = 0, limit = 0;  // held; more than limit (0: none) fails as a failed cudaMalloc does
     template <typename T>
     T* get(size_t count) {
         void* q = nullptr;
-        if (cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) return nullptr;
+        const size_t size = std::max<size_t>(count, 1) * sizeof(T);
+        if ((limit && bytes + size > limit) || cudaMalloc(&q, size) != cudaSuccess) {
+            cudaGetLastError();  // reported by the null pointer
+            return nullptr;
+        }
+        bytes += size;
         p.push_back(q);
         return (T*)q;
+    }
+    // frees what was allocated after p had `count` entries
+    void release(size_t count, size_t held) {
+        for (size_t k = count; k < p.size(); k++) cudaFree(p[k]);
+        p.resize(count);
+        bytes = held;
     }
     template <typename T>
     T* up(const T* h, size_t count) {
@@ -848,29 +860,36 @@ bool upload_window(lina_gpu_ilu* h, Factor& f, const WinPlan& pl, bool has_dinv)
 //   1025 x 1025 nodes, FP32: one block 2.87 ms, strips 0.52 ms
 //    389 x 389 nodes, FP64: one block 1.20 ms, strips 0.45 ms
 struct SolvePlan {
+    int n = 0;
+    std::vector<int> order, lev, lp, beg, end;  // levels and row segments
+    const int* col = nullptr;
+    bool has_dinv = false, lower = false;
     strip::Plan strips;
     WinPlan window;
     bool use32 = false, use64 = false;  // the strips are used in that precision
 };
 
-void plan_solve(SolvePlan& pl, int n, const std::vector<int>& order, const std::vector<int>& lev,
-                const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end, const int* col,
-                bool has_dinv, bool lower) {
-    const bool plan = strip::make_plan(pl.strips, n, order, lev, (int)lp.size() - 1, beg, end, col, lower);
+void plan_one_block(SolvePlan& pl) {
+    plan_window(pl.window, pl.n, pl.order, pl.lev, pl.lp, pl.beg, pl.end, pl.col, pl.has_dinv);
+}
+
+void plan_solve(SolvePlan& pl) {
+    const bool plan = strip::make_plan(pl.strips, pl.n, pl.order, pl.lev, (int)pl.lp.size() - 1, pl.beg, pl.end, pl.col,
+                                       pl.lower);
     pl.use32 = plan && strip::pays(pl.strips, false);
     pl.use64 = plan && strip::pays(pl.strips, true);
     if (pl.use32 && pl.use64) return;
-    plan_window(pl.window, n, order, lev, lp, beg, end, col, has_dinv);
+    plan_one_block(pl);
     if (!plan) return;
     pl.use32 = pl.use32 || !pl.window.w.s32;
     pl.use64 = pl.use64 || !pl.window.w.s64;
     if (!pl.use32 && !pl.use64) pl.strips = strip::Plan();
 }
 
-bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl, bool has_dinv) {
+bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl) {
     const strip::Plan& p = pl.strips;
     if (!p.strips || !pl.use32 || !pl.use64)
-        if (!upload_window(h, f, pl.window, has_dinv)) return false;
+        if (!upload_window(h, f, pl.window, pl.has_dinv)) return false;
     if (!p.strips) return true;
     Factor::Strips& w = f.strip;
     Mem& m = h->mem;
@@ -906,12 +925,47 @@ bool upload_solve(lina_gpu_ilu* h, Factor& f, const SolvePlan& pl, bool has_dinv
     return true;
 }
 
-bool build_solve(lina_gpu_ilu* h, Factor& f, int n, const std::vector<int>& order, const std::vector<int>& lev,
-                 const std::vector<int>& lp, const std::vector<int>& beg, const std::vector<int>& end,
-                 const int* col, bool has_dinv, bool lower) {
-    SolvePlan pl;
-    plan_solve(pl, n, order, lev, lp, beg, end, col, has_dinv, lower);
-    return upload_solve(h, f, pl, has_dinv);
+bool upload_factor(lina_gpu_ilu* h, const strip::Plan& p, const strip::FactorPlan& fplan) {
+    lina_gpu_ilu::StripFactor& w = h->sf;
+    Mem& m = h->mem;
+    w.used = fplan.used;
+    w.ring = p.ring;
+    w.strips = p.strips;
+    w.npos = (int)p.positions();
+    w.ext_first = m.up(fplan.ext_first);
+    w.ext = m.up(fplan.ext);
+    w.ext_end = m.up(fplan.ext_end);
+    w.rec = m.up(fplan.rec);
+    w.place = m.up(fplan.place);
+    w.a = m.get<double>((size_t)w.npos * (2 * fplan.width + 1));
+    if (!w.ext_first || !w.ext || !w.ext_end || !w.rec || !w.place || !w.a) return false;
+    w.width = fplan.width;
+    return true;
+}
+
+// The plans of both factors (and of the factorisation, fplan may be null) on the device, after everything else a
+// handle holds.  The strips' arrays take about 200 bytes a row more than the one-block solve's and the row pool's on mesh
+// matrices, several KB where levels have one row (a step holds 32): where they do not fit, in memory or in the
+// limit of lina_gpu_set_device_memory_limit, the handle does without them.
+bool upload_solves(lina_gpu_ilu* h, SolvePlan& L, SolvePlan& U, const strip::FactorPlan* fplan) {
+    Mem& m = h->mem;
+    const size_t count = m.p.size(), held = m.bytes;
+    const bool strips = L.strips.strips || U.strips.strips;
+    m.limit = strips ? (size_t)lina::dev::memory_limit() : 0;
+    const bool ok = upload_solve(h, h->L, L) && upload_solve(h, h->U, U) &&
+                    (!fplan || !fplan->width || upload_factor(h, L.strips, *fplan));
+    m.limit = 0;
+    if (ok || !strips) return ok;
+    m.release(count, held);
+    h->npos = 0;
+    h->L.strip = h->U.strip = Factor::Strips();
+    h->L.win = h->U.win = Factor::Win();
+    h->sf = lina_gpu_ilu::StripFactor();
+    for (SolvePlan* pl : {&L, &U}) {
+        pl->strips = strip::Plan();
+        plan_one_block(*pl);
+    }
+    return upload_solve(h, h->L, L) && upload_solve(h, h->U, U);
 }
 
 // the solve plan's packed copies of a factor's values and inverse diagonal (after every factorisation)
@@ -933,10 +987,11 @@ void pack_solve(Factor& f, int n) {
     }
 }
 
-// a factor given as CSR with its diagonal (lower: L with diagonal; upper: U, diagonal 1 skipped)
+// a factor given as CSR with its diagonal (lower: L with diagonal; upper: U, diagonal 1 skipped), without its solve;
+// col keeps the off-diagonal columns that the plan refers to
 bool build_factor(lina_gpu_ilu* h, Factor& f, int n, const int* p, const int* c, const double* v, bool lower,
-                  std::string& err) {
-    std::vector<int> ptr(n + 1, 0), col;
+                  SolvePlan& pl, std::vector<int>& col, std::string& err) {
+    std::vector<int> ptr(n + 1, 0);
     std::vector<double> val, dinv(n, 0.0);
     col.reserve(p[n]);
     val.reserve(p[n]);
@@ -969,12 +1024,15 @@ bool build_factor(lina_gpu_ilu* h, Factor& f, int n, const int* p, const int* c,
         dinv[i] = 1.0 / d;
         ptr[i + 1] = (int)col.size();
     }
-    std::vector<int> beg(ptr.begin(), ptr.end() - 1), end(ptr.begin() + 1, ptr.end()), order;
-    std::vector<int> lev, lp;
-    f.nlev = level_order(n, beg, end, col.data(), lower, order, &lev, &lp);
+    pl.n = n;
+    pl.beg.assign(ptr.begin(), ptr.end() - 1);
+    pl.end.assign(ptr.begin() + 1, ptr.end());
+    pl.col = col.data();
+    pl.lower = lower;
+    f.nlev = level_order(n, pl.beg, pl.end, pl.col, lower, pl.order, &pl.lev, &pl.lp);
     std::vector<float> val32(val.begin(), val.end()), dinv32(dinv.begin(), dinv.end());
     int* dptr = h->mem.up(ptr);
-    f.order = h->mem.up(order);
+    f.order = h->mem.up(pl.order);
     f.col = h->mem.up(col);
     f.val64 = h->mem.up(val);
     f.val32 = h->mem.up(val32);
@@ -991,11 +1049,8 @@ bool build_factor(lina_gpu_ilu* h, Factor& f, int n, const int* p, const int* c,
     }
     f.beg = dptr;
     f.end = dptr + 1;
-    if (!build_solve(h, f, n, order, lev, lp, beg, end, col.data(), !unit, lower)) {
-        err = "device allocation for the ILU factors failed";
-        return false;
-    }
-    pack_solve(f, n);
+    pl.has_dinv = !unit;
+    plan_solve(pl);
     return true;
 }
 
@@ -1224,13 +1279,18 @@ int lina_gpu_ilu_create(int n, const int* Lptr, const int* Lcol, const double* L
     lina_gpu_ilu* h = new lina_gpu_ilu();
     h->n = n;
     std::string err;
-    if (!lina::dev::ready() || !build_factor(h, h->L, n, Lptr, Lcol, Lval, true, err) ||
-        !build_factor(h, h->U, n, Uptr, Ucol, Uval, false, err) || !alloc_work(h)) {
+    SolvePlan lplan, uplan;
+    std::vector<int> lcol, ucol;
+    if (!lina::dev::ready() || !build_factor(h, h->L, n, Lptr, Lcol, Lval, true, lplan, lcol, err) ||
+        !build_factor(h, h->U, n, Uptr, Ucol, Uval, false, uplan, ucol, err) || !alloc_work(h) ||
+        !upload_solves(h, lplan, uplan, nullptr)) {
         g_ilu_err = err.empty() ? "device allocation failed" : err;
         lina::dev::set_error(("ILU: " + g_ilu_err).c_str());
         delete h;
         return LINA_GPU_EINVAL;
     }
+    pack_solve(h->L, n);
+    pack_solve(h->U, n);
     *out = h;
     return 0;
 }
@@ -1275,16 +1335,20 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
     lina_gpu_ilu* h = new lina_gpu_ilu();
     h->n = n;
     h->fnnz = nnz;
-    std::vector<int> lorder, uorder, llev, ulev, llp, ulp;
     lap("pattern checks and splits");
     // the level schedules and solve plans of L and U are independent: U's on a second thread
     SolvePlan lplan, uplan;
-    std::thread upper([&] {
-        h->U.nlev = level_order(n, ubeg, uend, col, false, uorder, &ulev, &ulp);
-        plan_solve(uplan, n, uorder, ulev, ulp, ubeg, uend, col, false, false);
-    });
-    h->L.nlev = level_order(n, lbeg, lend, col, true, lorder, &llev, &llp);
-    plan_solve(lplan, n, lorder, llev, llp, lbeg, lend, col, true, true);
+    auto plan = [&](SolvePlan& pl, Factor& f, std::vector<int>& beg, std::vector<int>& end, bool lower) {
+        pl.n = n;
+        pl.beg.swap(beg);
+        pl.end.swap(end);
+        pl.col = col;
+        pl.has_dinv = pl.lower = lower;
+        f.nlev = level_order(n, pl.beg, pl.end, col, lower, pl.order, &pl.lev, &pl.lp);
+        plan_solve(pl);
+    };
+    std::thread upper([&] { plan(uplan, h->U, ubeg, uend, false); });
+    plan(lplan, h->L, lbeg, lend, true);
     strip::FactorPlan fplan;
     strip::make_factor_plan(fplan, lplan.strips, n, rowptr, col, diag);
     upper.join();
@@ -1299,12 +1363,12 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
         ddiag = m.up(diag);
         dval = m.up(val, (size_t)nnz);
         h->fval = m.get<double>(nnz);
-        h->L.order = m.up(lorder);
-        h->U.order = m.up(uorder);
-        h->L.beg = m.up(lbeg);
-        h->L.end = m.up(lend);
-        h->U.beg = m.up(ubeg);
-        h->U.end = m.up(uend);
+        h->L.order = m.up(lplan.order);
+        h->U.order = m.up(uplan.order);
+        h->L.beg = m.up(lplan.beg);
+        h->L.end = m.up(lplan.end);
+        h->U.beg = m.up(uplan.beg);
+        h->U.end = m.up(uplan.end);
         h->L.dinv64 = m.get<double>(n);
         h->L.dinv32 = m.get<float>(n);
         h->L.val32 = m.get<float>(nnz);
@@ -1320,36 +1384,13 @@ int lina_gpu_ilu_create_from_matrix(int n, const int* rowptr, const int* col, co
     h->L.col = h->U.col = dcol;
     h->L.val64 = h->U.val64 = h->fval;
     h->U.val32 = h->L.val32;
-    if (!upload_solve(h, h->L, lplan, true) || !upload_solve(h, h->U, uplan, false)) {
-        lina::dev::set_error("ILU: device allocation failed");
-        delete h;
-        return LINA_GPU_ECUDA;
-    }
-    if (fplan.width) {
-        lina_gpu_ilu::StripFactor& w = h->sf;
-        w.width = fplan.width;
-        w.used = fplan.used;
-        w.ring = lplan.strips.ring;
-        w.strips = lplan.strips.strips;
-        w.npos = (int)lplan.strips.positions();
-        w.ext_first = m.up(fplan.ext_first);
-        w.ext = m.up(fplan.ext);
-        w.ext_end = m.up(fplan.ext_end);
-        w.rec = m.up(fplan.rec);
-        w.place = m.up(fplan.place);
-        w.a = m.get<double>((size_t)w.npos * (2 * w.width + 1));
-        if (!w.ext_first || !w.ext || !w.ext_end || !w.rec || !w.place || !w.a) {
-            lina::dev::set_error("ILU: device allocation failed");
-            delete h;
-            return LINA_GPU_ECUDA;
-        }
-    }
     h->flag = m.get<int>(n);
     h->aptr = dptr;
     h->acol = dcol;
     h->adiag = ddiag;
     h->aval = dval;
-    if (!h->flag || cudaMemsetAsync(h->flag, 0, (size_t)n * sizeof(int), st()) != cudaSuccess) {
+    if (!h->flag || cudaMemsetAsync(h->flag, 0, (size_t)n * sizeof(int), st()) != cudaSuccess ||
+        !upload_solves(h, lplan, uplan, &fplan)) {
         lina::dev::set_error("ILU: device allocation failed");
         delete h;
         return LINA_GPU_ECUDA;

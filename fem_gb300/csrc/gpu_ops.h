@@ -24,6 +24,7 @@ bool xpay(double* y, const double* x, double a, long n);  // y = x + a y
 bool sync();
 void* stream();                                    // the cudaStream_t used by these helpers
 void set_error(const char* msg);                   // text returned by lina_gpu_last_error()
+long memory_limit();                               // device bytes a handle may hold, 0: no limit
 
 }  // namespace dev
 }  // namespace lina

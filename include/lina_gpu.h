@@ -472,7 +472,9 @@ int lina_gpu_set_pdl(int on);
 /* Device bytes that one hierarchy or matrix handle may allocate (0, the default: no limit).  An allocation
    that would exceed it fails as a failed cudaMalloc does: the call returns LINA_GPU_ECUDA with the reason
    in lina_gpu_last_error(), frees what the handle holds, and the device stays usable.  For callers with a
-   fixed memory budget, and for tests of the failure paths. */
+   fixed memory budget, and for tests of the failure paths.  ILU handles are not refused: those created under a
+   limit that their fastest solve's arrays would exceed (about 400 bytes a row on mesh matrices) take the
+   solves that need less, with the same results. */
 int lina_gpu_set_device_memory_limit(long bytes);
 
 /* Dense inverse of a row-major m x m matrix in device memory, in place, by blocked Gauss-Jordan

@@ -101,3 +101,56 @@ def test_gpu_one_precision_on_strips(shape):
         assert np.abs(z - ref).max() <= 1e-13 * np.abs(ref).max()
         assert np.linalg.norm(z32 - ref) <= 1e-5 * np.linalg.norm(ref)
         assert np.array_equal(ilu.apply(r), z) and np.array_equal(ilu.apply(r, lina.PREC_MIXED), z32)
+
+
+@gpu
+@pytest.mark.gpu
+@pytest.mark.parametrize("make", [lambda: grid(1, 700), lambda: grid(31), lambda: grid(97), lambda: grid(300),
+                                  lambda: lines(3, 120, 400, 4),
+                                  lambda: (sp.kron(grid(40), np.ones((2, 2))) + 20 * sp.identity(3200)).tocsr()])
+def test_gpu_handles_without_memory_for_the_strips(make):
+    """Where the strips' arrays do not fit, a handle takes the one-block solve and the row pool: same factors, same
+    solutions, bit for bit, and less memory."""
+    torch = pytest.importorskip("torch")
+    A = make()
+    n = A.shape[0]
+    r = np.random.default_rng(6).standard_normal(n)
+    out, held = [], []
+    for limit in (0, 1):
+        free = torch.cuda.mem_get_info()[0]
+        lina.set_device_memory_limit(limit)
+        try:
+            ilu = lina.ILU(n, A.indptr, A.indices, A.data)
+        finally:
+            lina.set_device_memory_limit(0)
+        held.append(free - torch.cuda.mem_get_info()[0])
+        f = ilu.factor_values()
+        ilu.refactor(0.5 * A.data)
+        out.append([f, ilu.factor_values(), ilu.apply(r), ilu.apply(r, lina.PREC_MIXED)])
+        ilu.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+    if n >= 90000:
+        assert held[1] < held[0]
+    L, U = sp.tril(A, format="csr"), (sp.triu(A, 1) + sp.identity(n)).tocsr()
+    z = []
+    for limit in (0, 1):
+        lina.set_device_memory_limit(limit)
+        try:
+            z.append(factors(L, U, r))
+        finally:
+            lina.set_device_memory_limit(0)
+    assert np.array_equal(*z)
+
+
+def factors(L, U, r):
+    """U^-1 L^-1 r by a handle made from given factors."""
+    h, p = C.c_void_p(), lambda a: a.ctypes.data_as(C.c_void_p)
+    a = [np.ascontiguousarray(v) for T in (L, U) for v in (T.indptr.astype(np.int32), T.indices.astype(np.int32), T.data)]
+    fn = lina.lib().lina_gpu_ilu_create
+    fn.argtypes, fn.restype = [C.c_int] + [C.c_void_p] * 7, C.c_int
+    assert fn(len(r), *[p(v) for v in a], C.addressof(h)) == 0, lina.last_error()
+    x, z = lina.DeviceArray.from_host(r), lina.DeviceArray(len(r))
+    assert lina.lib().lina_gpu_ilu_apply(h, lina.PREC_FP64, x.ptr, z.ptr) == 0
+    out = z.to_host()
+    lina.lib().lina_gpu_ilu_destroy(h)
+    return out
