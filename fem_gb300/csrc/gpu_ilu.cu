@@ -1081,8 +1081,23 @@ __global__ void strip_rows_kernel(int npos, const int2* __restrict__ rec, const 
     }
 }
 
+// A probe of the waits: the strips from the first one on run without those before it, so that the entries they
+// fetch are never published, and give up after limit_ns.
+struct Probe {
+    int first = 0;
+    unsigned long long limit_ns = kWaitNs;
+};
+
+// the next kernel takes strips from p.first on
+void set_ticket(lina_gpu_ilu* h, const Probe& p) {
+    if (p.first == 0)
+        cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
+    else
+        fill_kernel<unsigned><<<1, 1, 0, st()>>>(1, (unsigned)p.first, h->ticket);
+}
+
 template <int W>
-void launch_strip_factor(lina_gpu_ilu* h) {
+void launch_strip_factor(lina_gpu_ilu* h, const Probe& probe) {
     const lina_gpu_ilu::StripFactor& w = h->sf;
     strip::FactorArgs a;
     a.ring = w.ring;
@@ -1098,6 +1113,7 @@ void launch_strip_factor(lina_gpu_ilu* h) {
     a.f = h->fval;
     a.ticket = h->ticket;
     a.err = h->err;
+    a.limit_ns = probe.limit_ns;
     static bool attr = false;
     if (!attr) {
         cudaFuncSetAttribute(strip::factor_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, strip::kSmemMax);
@@ -1105,7 +1121,17 @@ void launch_strip_factor(lina_gpu_ilu* h) {
     }
     strip_rows_kernel<W><<<std::min(4096, (w.npos + kT - 1) / kT), kT, 0, st()>>>(w.npos, a.rec, h->aval, w.a);
     cudaMemsetAsync(h->fval, 0xff, (size_t)h->fnnz * sizeof(double), st());  // every entry pending
-    strip::factor_kernel<W><<<w.strips, strip::factor_threads(W), strip::factor_smem(W, w.ring, a.stages), st()>>>(a);
+    set_ticket(h, probe);
+    strip::factor_kernel<W><<<w.strips - probe.first, strip::factor_threads(W), strip::factor_smem(W, w.ring, a.stages), st()>>>(a);
+}
+
+void strip_factorise(lina_gpu_ilu* h, const Probe& probe) {
+    switch (h->sf.width) {
+        case 1: launch_strip_factor<1>(h, probe); break;
+        case 2: launch_strip_factor<2>(h, probe); break;
+        case 3: launch_strip_factor<3>(h, probe); break;
+        default: launch_strip_factor<4>(h, probe); break;
+    }
 }
 
 // ILU(0) of the handle's A (pattern and values on the device) into fval, the inverse diagonal and
@@ -1114,14 +1140,11 @@ int factorise(lina_gpu_ilu* h) {
     const int n = h->n;
     const long nnz = h->fnnz;
     h->epoch++;
-    cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
-    switch (h->sf.width) {
-        case 1: launch_strip_factor<1>(h); break;
-        case 2: launch_strip_factor<2>(h); break;
-        case 3: launch_strip_factor<3>(h); break;
-        case 4: launch_strip_factor<4>(h); break;
-        default:
-            ilu0_kernel<<<pool_blocks(n), kPool, 0, st()>>>(n, h->L.order, h->aptr, h->acol, h->aval, h->adiag, h->U.beg,
+    if (h->sf.width) {
+        strip_factorise(h, Probe());
+    } else {
+        cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
+        ilu0_kernel<<<pool_blocks(n), kPool, 0, st()>>>(n, h->L.order, h->aptr, h->acol, h->aval, h->adiag, h->U.beg,
                                                             h->fval, h->flag, h->epoch, h->ticket, h->err);
     }
     diag_inverse_kernel<<<std::min(4096, (n + kT - 1) / kT), kT, 0, st()>>>(n, h->adiag, h->fval, h->L.dinv64,
@@ -1180,7 +1203,7 @@ void launch_strips(const strip::Args<TX>& a, int strips, size_t smem, bool dinv)
 
 // the solve pipelined over strips; the right-hand side may be wider than the solve's type
 template <typename TX, typename TB>
-void solve_strips(lina_gpu_ilu* h, const Factor& f, const TX* dinv, const TB* b, TX* x) {
+void solve_strips(lina_gpu_ilu* h, const Factor& f, const TX* dinv, const TB* b, TX* x, const Probe& probe = Probe()) {
     const Factor::Strips& w = f.strip;
     strip::Args<TX> a;
     a.ring = w.ring;
@@ -1204,16 +1227,18 @@ void solve_strips(lina_gpu_ilu* h, const Factor& f, const TX* dinv, const TB* b,
     a.x = x;
     a.ticket = h->ticket;
     a.err = h->err;
+    a.limit_ns = probe.limit_ns;
     gather_pos_kernel<TB, TX><<<std::min(4096, (w.npos + kT - 1) / kT), kT, 0, st()>>>(w.npos, w.row, b, bpos);
     cudaMemsetAsync(x, 0xff, (size_t)h->n * sizeof(TX), st());  // every entry pending
-    cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), st());
+    set_ticket(h, probe);
     const size_t smem = strip::smem_bytes(w.ring, w.max_width, sizeof(TX), a.stages);
+    const int blocks = w.strips - probe.first;
     switch (w.width) {
-        case 1: launch_strips<TX, 1>(a, w.strips, smem, dinv != nullptr); break;
-        case 2: launch_strips<TX, 2>(a, w.strips, smem, dinv != nullptr); break;
-        case 3: launch_strips<TX, 3>(a, w.strips, smem, dinv != nullptr); break;
-        case 4: launch_strips<TX, 4>(a, w.strips, smem, dinv != nullptr); break;
-        default: launch_strips<TX, 0>(a, w.strips, smem, dinv != nullptr); break;
+        case 1: launch_strips<TX, 1>(a, blocks, smem, dinv != nullptr); break;
+        case 2: launch_strips<TX, 2>(a, blocks, smem, dinv != nullptr); break;
+        case 3: launch_strips<TX, 3>(a, blocks, smem, dinv != nullptr); break;
+        case 4: launch_strips<TX, 4>(a, blocks, smem, dinv != nullptr); break;
+        default: launch_strips<TX, 0>(a, blocks, smem, dinv != nullptr); break;
     }
 }
 
@@ -1446,6 +1471,50 @@ int lina_gpu_wait_probe(int limit_us, double* waited_us) {
     if (waited_us) *waited_us = ns / 1000.0;
     if (e != 0) {
         lina::dev::set_error("a device wait ran out (no row ever published the awaited value)");
+        return LINA_GPU_ECUDA;
+    }
+    return 0;
+}
+
+// The failure path of the strips' own waits, made to happen on a handle: the strips of L but the first run as in a
+// solve (what = LINA_PREC_FP64 or LINA_PREC_MIXED) or in the factorisation (what = 2), and wait up to limit_us
+// for entries of the first that nothing publishes.  Returns LINA_GPU_ECUDA with the error text set, the time taken
+// in *waited_us, the handle usable (its factors formed again); LINA_GPU_EINVAL where it has fewer than two strips.
+int lina_gpu_ilu_wait_probe(lina_gpu_ilu* h, int what, int limit_us, double* waited_us) {
+    if (!h || limit_us <= 0 || limit_us > 1000000) return LINA_GPU_EINVAL;
+    const bool factor = what == 2;
+    const bool on = factor ? h->sf.width > 0 : what == LINA_PREC_MIXED ? h->L.strip.use32 : h->L.strip.use64;
+    if ((!factor && what != LINA_PREC_FP64 && what != LINA_PREC_MIXED) || !on || h->L.strip.strips < 2)
+        return LINA_GPU_EINVAL;
+    const Probe probe{1, 1000ull * (unsigned long long)limit_us};
+    const int g = std::min(4096, (h->n + kT - 1) / kT);
+    if (cudaStreamSynchronize(st()) != cudaSuccess) return LINA_GPU_ECUDA;
+    const auto t0 = std::chrono::steady_clock::now();
+    if (factor) {
+        strip_factorise(h, probe);
+    } else if (what == LINA_PREC_MIXED) {
+        fill_kernel<float><<<g, kT, 0, st()>>>(h->n, 1.0f, h->r32);
+        solve_strips<float, float>(h, h->L, h->L.dinv32, h->r32, h->t32, probe);
+    } else {
+        Mem m;
+        double* b = m.get<double>(h->n);
+        if (!b) return LINA_GPU_ECUDA;
+        fill_kernel<double><<<g, kT, 0, st()>>>(h->n, 1.0, b);
+        solve_strips<double, double>(h, h->L, h->L.dinv64, b, h->t64, probe);
+        if (cudaStreamSynchronize(st()) != cudaSuccess) return LINA_GPU_ECUDA;
+    }
+    if (cudaGetLastError() != cudaSuccess) return LINA_GPU_ECUDA;
+    const int e = read_err(h);
+    if (waited_us)
+        *waited_us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();
+    if (e < 0) return LINA_GPU_ECUDA;
+    cudaMemset(h->err, 0, sizeof(int));
+    if (factor) {
+        const int rc = factorise(h);
+        if (rc) return rc;
+    }
+    if (e != 0) {
+        lina::dev::set_error("ILU: a wait of the strips ran out (no row ever published the awaited value)");
         return LINA_GPU_ECUDA;
     }
     return 0;

@@ -45,6 +45,7 @@ struct FactorArgs {
     double* f;                 // CSR entry -> factor value, the pending pattern on entry
     unsigned* ticket;
     int* err;                  // 1 a wait ran out, 2 zero pivot
+    unsigned long long limit_ns;  // of every wait
 };
 
 struct FactorStage {
@@ -113,12 +114,12 @@ __global__ void __launch_bounds__(factor_threads(W), 1) factor_kernel(const Fact
     const int c0 = __ldg(a.first + strip), c1 = __ldg(a.first + strip + 1);
     if (warp > W + 1) {
         fetch_entries<double>(a.f, a.ext, __ldg(a.ext_first + strip), __ldg(a.ext_first + strip + 1),
-                              threadIdx.x - 32 * (W + 2), slots, a.err);
+                              threadIdx.x - 32 * (W + 2), slots, a.err, a.limit_ns);
         return;
     }
     if (warp == W + 1) {
         if (lane != 0) return;
-        copy_chunks(c0, c1, a.stages, L.bytes, stages, bars, ctl + 1, a.err, [&](int c, unsigned char* st, uint64_t* bar) {
+        copy_chunks(c0, c1, a.stages, L.bytes, stages, bars, ctl + 1, a.err, a.limit_ns, [&](int c, unsigned char* st, uint64_t* bar) {
             bulk::mbar_expect_tx(bar, (unsigned)L.bytes);
             bulk::copy(st + L.rec, a.rec + (size_t)c * kPos, 8u * kPos, bar);
             bulk::copy(st + L.place, a.place + (size_t)c * kPos * NP, 2u * kPos * NP, bar);
@@ -155,7 +156,7 @@ __global__ void __launch_bounds__(factor_threads(W), 1) factor_kernel(const Fact
     for (int c = 0; c < chunks; c++) {
         const unsigned char* st = stages + stage * L.bytes;
         bool ok = bulk::mbar_wait(bars + stage, phase, a.err, 1);
-        ok = await_entries<double>(got, end, first, slots, lane, a.err) && ok;
+        ok = await_entries<double>(got, end, first, slots, lane, a.err, a.limit_ns) && ok;
         if (!walkers_all<W>(ok)) break;
         for (int i = 0; i < kSteps; i++) {
             const int p = 32 * i + lane;

@@ -124,6 +124,7 @@ struct Args {
     TX* x;                  // row -> solution, the pending pattern on entry
     unsigned* ticket;       // strips taken, 0 on entry
     int* err;
+    unsigned long long limit_ns;  // of every wait
 };
 
 // byte offsets inside a stage, for chunks of up to `width` entries per row
@@ -150,11 +151,12 @@ inline int stages_for(int ring, int width, int tx) {
 }
 
 // after a failed poll: every 64th looks at the error word and the clock (a read of either costs as much as
-// the wait); false: give up
-__device__ __forceinline__ bool keep_waiting(long& polls, unsigned long long& t0, int* err, int code) {
+// the wait); false: give up (after limit_ns)
+__device__ __forceinline__ bool keep_waiting(long& polls, unsigned long long& t0, int* err, int code,
+                                             unsigned long long limit_ns) {
     if ((++polls & 63) != 0) return true;
     if (polls == 64) t0 = bulk::device_ns();
-    if (polls > bulk::kWaitPolls || *(volatile int*)err || bulk::device_ns() - t0 > bulk::kWaitNs) {
+    if (polls > bulk::kWaitPolls || *(volatile int*)err || bulk::device_ns() - t0 > limit_ns) {
         atomicCAS(err, 0, code);
         return false;
     }
@@ -165,7 +167,7 @@ __device__ __forceinline__ bool keep_waiting(long& polls, unsigned long long& t0
 // slot is empty.  One loop for all lanes, each at an entry of its own: a lane that waits holds up no other.
 template <typename TX>
 __device__ void fetch_entries(const TX* x, const int* __restrict__ ext, int e0, int e1, int lane, unsigned char* slots,
-                              int* err) {
+                              int* err, unsigned long long limit_ns) {
     using B = Bits<TX>;
     using U = typename B::U;
     int e = e0 + lane;
@@ -184,7 +186,7 @@ __device__ void fetch_entries(const TX* x, const int* __restrict__ ext, int e0, 
             src = nsrc;
             nsrc = e + 32 * kHelpers < e1 ? __ldg(ext + e + 32 * kHelpers) : 0;
             polls = 0;
-        } else if (!keep_waiting(polls, t0, err, 1)) {
+        } else if (!keep_waiting(polls, t0, err, 1, limit_ns)) {
             return;
         }
     }
@@ -194,14 +196,14 @@ __device__ void fetch_entries(const TX* x, const int* __restrict__ ext, int e0, 
 // per lane, looked at before; where all were there and they are at most 32, nothing is waited for.
 template <typename TX>
 __device__ __forceinline__ bool await_entries(int got, int end, typename Bits<TX>::U first, const unsigned char* slots,
-                                              int lane, int* err) {
+                                              int lane, int* err, unsigned long long limit_ns) {
     bool ok = true;
     if (end - got > 32 || __any_sync(0xffffffffu, first == Bits<TX>::kPending)) {
         for (int e = got + lane; e < end; e += 32) {
             const unsigned char* slot = slots + e % kSlots * (int)sizeof(TX);
             long polls = 0;
             unsigned long long t0 = 0;
-            while (ok && get<TX>(slot) == Bits<TX>::kPending) ok = keep_waiting(polls, t0, err, 1);
+            while (ok && get<TX>(slot) == Bits<TX>::kPending) ok = keep_waiting(polls, t0, err, 1, limit_ns);
         }
         __syncwarp();
     }
@@ -212,13 +214,13 @@ __device__ __forceinline__ bool await_entries(int got, int end, typename Bits<TX
 // with chunk c - S; issue(c, stage, barrier) announces the chunk's bytes and starts its copies
 template <typename F>
 __device__ __forceinline__ void copy_chunks(int c0, int c1, int S, int stage_bytes, unsigned char* stages, uint64_t* bars,
-                                            const volatile int* done, int* err, F issue) {
+                                            const volatile int* done, int* err, unsigned long long limit_ns, F issue) {
     int c = c0;
     for (; c < c1; c++) {
         long polls = 0;
         unsigned long long t0 = 0;
         bool ok = true;
-        while (ok && *done < c - c0 - S + 1) ok = keep_waiting(polls, t0, err, 1);
+        while (ok && *done < c - c0 - S + 1) ok = keep_waiting(polls, t0, err, 1, limit_ns);
         if (!ok) break;
         bulk::fence_proxy_async();  // the stage was last read through ordinary loads
         issue(c, stages + ((c - c0) % S) * stage_bytes, bars + (c - c0) % S);
@@ -255,12 +257,12 @@ __global__ void __launch_bounds__(kThreads, 1) solve_kernel(const Args<TX> a) {
     const int c0 = __ldg(a.first + strip), c1 = __ldg(a.first + strip + 1);
     if (warp >= 2) {
         fetch_entries<TX>(a.x, a.ext, __ldg(a.ext_first + strip), __ldg(a.ext_first + strip + 1), threadIdx.x - 64, slots,
-                          a.err);
+                          a.err, a.limit_ns);
         return;
     }
     if (warp == 1) {
         if (lane != 0) return;
-        copy_chunks(c0, c1, a.stages, L.bytes, stages, bars, ctl + 1, a.err, [&](int c, unsigned char* st, uint64_t* bar) {
+        copy_chunks(c0, c1, a.stages, L.bytes, stages, bars, ctl + 1, a.err, a.limit_ns, [&](int c, unsigned char* st, uint64_t* bar) {
             const int4 tb = __ldg(a.table + c);
             const unsigned pb = (unsigned)sizeof(TX) * kPos;
             bulk::mbar_expect_tx(bar, pb * (3u + 2u * tb.y));
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) solve_kernel(const Args<TX> a) {
             nphase ^= 1u;
         }
         const int w = EM > 0 ? EM : __ldg(a.table + c0 + c).y;
-        ok = await_entries<TX>(got, end, first, slots, lane, a.err) && ok;
+        ok = await_entries<TX>(got, end, first, slots, lane, a.err, a.limit_ns) && ok;
 #pragma unroll
         for (int i = 0; i < kSteps; i++) {
             U res;

@@ -237,6 +237,11 @@ int lina_gpu_ilu_destroy(lina_gpu_ilu* h);
    LINA_GPU_ECUDA with the error text a timed-out solve gives, and the time waited in *waited_us;
    the device stays usable.  For tests of the library's failure handling. */
 int lina_gpu_wait_probe(int limit_us, double* waited_us);
+/* The same for the waits of the solves and the factorisation pipelined over strips of rows, on a handle: the
+   strips of L but the first run in the solve of a precision (what = LINA_PREC_FP64 or LINA_PREC_MIXED) or in the
+   factorisation (what = 2) and wait up to limit_us for what the first never publishes.  LINA_GPU_ECUDA with the
+   error text, as above; the handle stays usable.  LINA_GPU_EINVAL where it has fewer than two strips. */
+int lina_gpu_ilu_wait_probe(lina_gpu_ilu* h, int what, int limit_us, double* waited_us);
 int lina_gpu_ilu_levels(const lina_gpu_ilu* h, int* nlev_L, int* nlev_U);
 /* z = U^-1 L^-1 r (device vectors, FP64); LINA_PREC_MIXED solves in FP32 */
 int lina_gpu_ilu_apply(lina_gpu_ilu* h, int precision, const double* r_dev, double* z_dev);
