@@ -1,4 +1,6 @@
-// Which solve a triangular factor takes (strip_plan.h): the strips' plan, its estimates and the choice by them.
+// Which solve a triangular factor takes (strip_plan.h): the strips' plan, its estimates and the choice by them; and
+// the row recurrence, each product and sum rounded as one fused operation.
+#include <cmath>
 #include <vector>
 
 #include "strip_plan.h"
@@ -21,4 +23,23 @@ extern "C" int strip_rules(int n, const int* ptr, const int* col, int lower, dou
     const double v[] = {double(P.strips), double(P.width), double(P.max_width), P.ns32, P.win32, P.ns64, P.win64};
     for (int k = 0; k < 7; k++) out[k] = v[k];
     return (strip::pays(P, false) ? 1 : 0) | (strip::pays(P, true) ? 2 : 0);
+}
+
+template <typename T>
+static void recurrence(int n, const int* ptr, const int* col, const T* val, const T* dinv, int lower, const T* b, T* x) {
+    for (int t = 0; t < n; t++) {
+        const int i = lower ? t : n - 1 - t;
+        T s = b[i];
+        for (int p = ptr[i]; p < ptr[i + 1]; p++) s = std::fma(-val[p], x[col[p]], s);
+        x[i] = dinv ? s * dinv[i] : s;
+    }
+}
+
+extern "C" void recurrence64(int n, const int* ptr, const int* col, const double* val, const double* dinv, int lower,
+                             const double* b, double* x) {
+    recurrence(n, ptr, col, val, dinv, lower, b, x);
+}
+extern "C" void recurrence32(int n, const int* ptr, const int* col, const float* val, const float* dinv, int lower,
+                             const float* b, float* x) {
+    recurrence(n, ptr, col, val, dinv, lower, b, x);
 }
