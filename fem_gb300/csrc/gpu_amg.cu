@@ -3590,7 +3590,7 @@ int build_stage(lina_gpu_amg* h, DLevel& L, const lina::Csr& A, const Colours& c
     const StageSizes z = stage_sizes(A, colours, groups, K);
     if (z.bytes(4) > (size_t)kStagedSmemMax) return 0;
     const bool f64 = z.bytes(8) <= (size_t)kStagedSmemMax;
-    if (h->lean && !f64) return 0;
+    if (h->lean && !layout::lean_images(z.rows, C, z.pmax, z.emax)) return 0;
     // the FP64 lanes of every colour, from its largest share
     std::vector<int> lanes64(C, L.Acol.lanes64);
     std::vector<int> len;
@@ -5325,12 +5325,6 @@ int lina_gpu_batch_destroy(lina_gpu_batch* B) {
 // every system has stopped.
 namespace {
 
-// Rows per task of the segmented kernels: enough tasks for four blocks of 256 threads on each of the 152 SMs, of
-// at least four rows a thread (a task's reduction costs as much as some rows) and at most 4,096.  16 systems of
-// 608,657 rows in all, tasks of 1,024 rows with all loads of two or four rows in flight (before: 157 tasks of 4,096,
-// a row at a time): r.z and z.q_j 16.2 us (28.9), p 11.9 (22.3), x and r 8.1 (18.6), p.q 4.8 (8.9).
-int seg_chunk(int n) { return std::min(4096, std::max(1024, (n / (4 * 152) + 255) / 256 * 256)); }
-
 struct SegScalars {
     double s, s_old, pq, alpha, rr, r0, tol, tnorm2;
     double tj[kFcgMax], pqh[kFcgMax], cj[kFcgMax];
@@ -5903,7 +5897,7 @@ int lina_gpu_segbatch_create(int count, lina_gpu_amg* const* systems, lina_gpu_s
         return rc;
     }
     B->off = map.off[c->depth - 1];
-    const int chunk = seg_chunk(B->off[count]);
+    const int chunk = layout::seg_chunk(B->off[count], c->lean);
     std::vector<int4> tasks;
     std::vector<int> tbeg(count + 1, 0);
     for (int i = 0; i < count; i++) {

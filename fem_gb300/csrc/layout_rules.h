@@ -163,4 +163,23 @@ inline int stage_lanes64(const std::vector<int>& len, int lanes, int asked) {
     return best;
 }
 
+// Whether a handle with a device-memory limit has images for the staged steps of a level (of `rows` rows and c
+// colours, the largest share of a block p rows and e entries): only where they would fit a block's 210 KB in FP64
+// with columns of 4 bytes and no masks.  The images themselves are smaller, so such a handle holds no more for them
+// than that size, and none for levels that only the smaller ones fit.
+inline bool lean_images(size_t rows, size_t c, size_t p, size_t e) {
+    auto pad = [](size_t v) { return (v + 3) / 4 * 4; };
+    const size_t ints = pad(c + 1) + pad(p) + pad(p + 1) + pad(e), values = pad(e) + 2 * pad(p);
+    return (rows * 8 + 15) / 16 * 16 + 8 * values + 4 * ints <= 210 * 1024;
+}
+
+// Rows per task of the segmented kernels: enough tasks for four blocks of 256 threads on each of the 152 SMs, of
+// at least four rows a thread (a task's reduction costs as much as some rows) and at most 4,096.  16 systems of
+// 608,657 rows in all, tasks of 1,024 rows with all loads of two or four rows in flight (before: 157 tasks of 4,096,
+// a row at a time): r.z and z.q_j 16.2 us (28.9), p 11.9 (22.3), x and r 8.1 (18.6), p.q 4.8 (8.9).  Handles with a
+// device-memory limit keep tasks of 4,096 rows, whose partials take a quarter of the memory.
+inline int seg_chunk(int n, bool lean) {
+    return lean ? 4096 : std::min(4096, std::max(1024, (n / (4 * 152) + 255) / 256 * 256));
+}
+
 }  // namespace layout

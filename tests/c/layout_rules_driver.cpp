@@ -20,3 +20,7 @@ extern "C" int rule_groups_allowed(int asked) { return layout::groups_allowed(as
 extern "C" int rule_sell_variant(int f64, int long_rows, long npos) {
     return (int)layout::sell_variant(f64 != 0, long_rows != 0, npos);
 }
+
+extern "C" int rule_lean_images(long rows, long c, long p, long e) { return layout::lean_images(rows, c, p, e) ? 1 : 0; }
+
+extern "C" int rule_seg_chunk(int n, int lean) { return layout::seg_chunk(n, lean != 0); }

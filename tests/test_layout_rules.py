@@ -111,6 +111,21 @@ def test_sell_variants_by_blocks_per_sm(rules):
     assert [v(0, 1, n) for n in (32, 38912, 38944, 1 << 20)] == [3, 3, 2, 2]
 
 
+def test_handles_with_a_memory_limit_hold_no_more(rules):
+    """Their staged images are bounded by what images with 4-byte columns took (8 rows + 12 entries + 24 p bytes and the
+    colours), their batches' tasks have 4,096 rows."""
+    f = rules.rule_lean_images
+    f.argtypes = [C.c_long] * 4
+    size = lambda rows, c, p, e: 8 * rows + 12 * e + 24 * p + 4 * (c + 1 + 3)  # noqa: E731
+    for c in (1, 4, 22):
+        for rows, p in ((16, 1), (1600, 100), (9216, 576), (20000, 1252)):
+            last = [e for e in range(0, 20000, 4) if f(rows, c, p, e)][-1]
+            assert abs(size(rows, c, p, last) - 210 * 1024) <= 128
+    # 9,216 rows of 14 entries over 16 blocks: 16-bit columns would fit, 4-byte columns do not
+    assert f(9216, 12, 576, 9000) and not f(9216, 12, 576, 10752)
+    assert [rules.rule_seg_chunk(n, lean) for n in (100, 608657, 5000000) for lean in (0, 1)] == [1024, 4096, 1024, 4096, 4096, 4096]
+
+
 def ring(n):
     """Periodic second differences with a shift."""
     e = np.ones(n)
