@@ -455,7 +455,8 @@ int lina_gpu_set_fused_groups(int on);
    at most 50M stored entries) in
    each candidate layout at upload (one thread per row, or 4, 8 or 16 lanes per row), 5 smoother sweeps
    plus a residual in their precision, and keep the fastest (default 0 = the fixed layout rule; segmented
-   batches always tune).  The choice depends on timings, so two hierarchies of one matrix may differ in
+   batches always tune the levels that they run colour by colour).  Staged multicolour-SOR steps choose their
+   FP64 lanes colour by colour whatever was tuned.  The choice depends on timings, so two hierarchies of one matrix may differ in
    layout and hence in rounding.  LINA_SETUP_TIMING prints the times. */
 int lina_gpu_set_autotune(int on);
 /* 16 (default): SELL-32 matrices with long rows (at least 24 stored entries per row on average)
