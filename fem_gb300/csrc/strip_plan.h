@@ -229,8 +229,8 @@ inline bool make_plan(Plan& P, int n, const std::vector<int>& order, const std::
     return true;
 }
 
-// Whether the strips are used where the one-block solve is there too.  Most mesh matrices gain 2 to 5 times in either
-// precision (5-, 7- and 9-point grids, Delaunay meshes, interleaved components).  Few do not: levels that cross few
+// Whether the strips are used where the one-block solve is there too.  Most mesh matrices gain 1.4 to 5 times in either
+// precision (5- to 13-point grids, Delaunay meshes, interleaved components).  Few do not: levels that cross few
 // strips, so that a strip walks several steps of each (four strips of 100 lines of 120 points, coupled to the
 // line before by e points: FP64 569 us one block, 656 strips for e = 3, 722 and 1,163 for 5, 1,003 and 2,174 for
 // 12; FP32 478 and 228, 557 and 677, 685 and 776).
